@@ -164,10 +164,14 @@ struct ProfileSystem {
   double *invD, *piv;      // [nt*32] reciprocal pivots, pivots
   const int4 *tasks;       // [ntasks] factor tasks (type, I, K, J) in dataflow order
   int ntasks;
-  int *next_task;          // [1] task counter
-  int *upd, *done;         // [nt*(W+1)] per tile: updates applied, factored
+  int *next_task;          // [2] task counter, block tickets
+  int *upd, *done;         // [nt*(W+1)] per tile: updates applied, finished
+  int *colcnt;             // [nt] tile pairs of each column applied
+  const int *npairs;       // [nt] tile pairs of each column
+  unsigned char *dig;      // ring of the panels' digits (profile_digit_bytes)
   double *sweep;           // [4*4*nt*32] values published by the sweeps (y, c, x, c')
-  int *flags;              // [4]
+  int *flags;              // [4]; the counters above follow it in one block
+  size_t counter_bytes;    // of that block
   double min_diag_tol;
   // per tile row J, for the substitutions (row-major 32 x 32 each,
   // [nt*1024]): W_J = L_JJ^-T, F_J = L_JJ^-1 L_J,J-1, G_J = L_JJ^-T
@@ -175,29 +179,36 @@ struct ProfileSystem {
   // Q_J = E_J - F_J F_J-1 and R_J = H_J - G_J G_J+1 (zero where a tile is
   // outside the envelope)
   double *Winv, *F, *G, *E, *H, *Q, *R;
-  int *cpl;                // [nt] row J's coupling matrices written
+  // [nt] row J's W written, its first four coupling matrices, its Q
+  int *cplw, *cpl, *cplq;
+  // columns published by the factorisation: [nt][column][row] of L_JJ (the
+  // reciprocal pivot on the diagonal), then [nt][column][P rows, L rows] of
+  // panel (J+1, J)
+  double *lstream, *wlstream;
   // right-hand sides whose forward sweep runs inside the factorisation
-  // (fwd_nrhs 0: none), column r at fwd_x[r*fwd_ldx]
-  int fwd_nrhs, fwd_ldx;
-  const double *fwd_x;
+  // (fwd_nrhs 0: none)
+  int fwd_nrhs;
+  const double *b[4];      // right-hand sides [n]
+  double *x[4];            // solutions [n]
 };
 int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &ftile, int &nt,
                  int &W);
-void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks);
+void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks,
+                   std::vector<int> &npairs);
 size_t profile_tile_doubles(int nt, int W);
+size_t profile_digit_bytes(int W);
 int profile_tile_edge();
-// Factor the CSR values into the tiles.  XG_ESOLVE on a failed pivot check
-// (*bad_eq = the equation) or a dependency wait that timed out (*bad_eq = -1).
-int profile_factor(const ProfileSystem &S, cudaStream_t s, int *bad_eq);
-// Solve in place: x[r*ldx + i] holds right-hand side r on entry (ldx >=
-// nt*32, entries past n zero), the solution on return; nrhs <= 4.
-// backward_only: the factorisation ran the forward sweep of these
-// right-hand sides (ProfileSystem::fwd_nrhs, the pipelined path only).
-int profile_solve(const ProfileSystem &S, int nrhs, double *x, int ldx, cudaStream_t s,
-                  bool backward_only = false);
-// Whether the substitutions of this system run pipelined over co-resident
-// blocks (the path whose forward sweep the factorisation can carry).
-bool profile_pipelined(const ProfileSystem &S);
+// Factor the CSR values into the tiles, with the forward sweep of
+// fwd_nrhs right-hand sides b.  Enqueued only; profile_status tells the
+// outcome.
+int profile_factor(const ProfileSystem &S, cudaStream_t s);
+// x[r] = A^-1 b[r] for r < nrhs <= 4 (x may be b).  backward_only: the
+// factorisation ran the forward sweep of these right-hand sides
+// (ProfileSystem::fwd_nrhs); after a failed one nothing is written.
+int profile_solve(const ProfileSystem &S, int nrhs, cudaStream_t s, bool backward_only = false);
+// Waits for the stream.  XG_ESOLVE on a failed pivot check (*bad_eq = the
+// equation) or a wait that timed out (*bad_eq = -1).
+int profile_status(const ProfileSystem &S, cudaStream_t s, int *bad_eq);
 
 // The tiled envelope LDL' with its device buffers: planned once per pattern,
 // factored once per tangent, then up to four right-hand sides per solve.
@@ -217,20 +228,15 @@ class ProfileSolver {
   int setup(int n, const int *rowptr, const int *colidx, const int *d_rowptr,
             const int *d_colidx, const double *d_vals, cudaStream_t s);
   bool ready() const { return ready_; }
-  // Factor the values now in d_vals.  XG_ESOLVE on a failed pivot check
-  // (*bad_eq = the equation) or a dependency wait that timed out (*bad_eq =
-  // -1).
-  int factor(cudaStream_t s, int *bad_eq);
-  // x[r] = A^-1 b[r] for r < nrhs (1..4; device vectors of n entries) with
-  // the last factorisation.
+  // Factor the values now in d_vals with the forward sweep of b[0..nrhs)
+  // running right behind its front (device vectors of n entries, 1..4 of
+  // them); solve_backward then finishes x[r] = A^-1 b[r] and returns the
+  // outcome of both: XG_ESOLVE on a failed pivot check (*bad_eq = the
+  // equation) or a dependency wait that timed out (*bad_eq = -1).
+  int factor_forward(int nrhs, const double *const *b, cudaStream_t s);
+  int solve_backward(int nrhs, double *const *x, cudaStream_t s, int *bad_eq);
+  // x[r] = A^-1 b[r] with the last factorisation.
   int solve(int nrhs, const double *const *b, double *const *x, cudaStream_t s);
-  // Factor with the forward sweep of b[0..nrhs) running as tasks of the
-  // factorisation (right behind its front); solve_backward then finishes
-  // x[r] = A^-1 b[r].  Only for systems whose substitutions are pipelined
-  // (can_fuse()).
-  bool can_fuse() const { return ready_ && profile_pipelined(S_); }
-  int factor_forward(int nrhs, const double *const *b, cudaStream_t s, int *bad_eq);
-  int solve_backward(int nrhs, double *const *x, cudaStream_t s);
   const ProfileSystem &system() const { return S_; }
 
  private:
@@ -243,9 +249,9 @@ class ProfileSolver {
   ProfileSystem S_{};
   int fwd_nrhs_ = 0;         // right-hand sides factor_forward swept
   bool ready_ = false;
-  int ldx_ = 0;
-  Buf<int> ftile_, flags_, tasks_, next_, upd_, done_, cpl_;
-  Buf<double> L_, invD_, piv_, px_, Winv_, F_, G_, E_, H_, Q_, R_, sweep_;
+  Buf<int> ftile_, counters_, tasks_, npairs_;
+  Buf<unsigned char> dig_;
+  Buf<double> L_, invD_, piv_, Winv_, F_, G_, E_, H_, Q_, R_, sweep_, stream_;
 };
 
 // ProfileSPD for many small disconnected parts, one band per part

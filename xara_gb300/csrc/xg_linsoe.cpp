@@ -318,9 +318,15 @@ static int linsoe_solve_profile(xg_linsoe *s, int *iters, double *relres) {
                       cudaMemcpyHostToDevice, st) != cudaSuccess)
     return lfail(XG_ECUDA, "xg_linsoe_solve: copy of A failed");
   s->prof_vals_stale = false;
+  const double *bp = s->b.p;
+  double *xp = s->x.p;
+  if (cudaMemcpyAsync(s->b.p, s->B.data(), s->B.size() * sizeof(double), cudaMemcpyHostToDevice,
+                      st) != cudaSuccess)
+    return lfail(XG_ECUDA, "xg_linsoe_solve: copy of B failed");
   if (!s->prof_factored) {
-    int bad = -1;
-    if (s->prof.factor(st, &bad) != 0) {
+    int bad = -1, e = s->prof.factor_forward(1, &bp, st);
+    if (!e) e = s->prof.solve_backward(1, &xp, st, &bad);
+    if (e) {
       char msg[160];
       if (bad >= 0)
         snprintf(msg, sizeof msg, "xg_linsoe_solve: ProfileSPD pivot %d fails the check (aii == "
@@ -330,13 +336,9 @@ static int linsoe_solve_profile(xg_linsoe *s, int *iters, double *relres) {
       return lfail(XG_ESOLVE, msg);
     }
     s->prof_factored = true;
+  } else if (int e = s->prof.solve(1, &bp, &xp, st)) {
+    return lfail(e, "xg_linsoe_solve: substitutions failed");
   }
-  const double *bp = s->b.p;
-  double *xp = s->x.p;
-  if (cudaMemcpyAsync(s->b.p, s->B.data(), s->B.size() * sizeof(double), cudaMemcpyHostToDevice,
-                      st) != cudaSuccess)
-    return lfail(XG_ECUDA, "xg_linsoe_solve: copy of B failed");
-  if (int e = s->prof.solve(1, &bp, &xp, st)) return lfail(e, "xg_linsoe_solve: substitutions failed");
   if (cudaMemcpyAsync(s->X.data(), s->x.p, s->n * sizeof(double), cudaMemcpyDeviceToHost, st) !=
           cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)

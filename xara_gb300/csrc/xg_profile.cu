@@ -1,40 +1,60 @@
 // xg_profile.cu -- the `system ProfileSPD` path on the device: LDL' of the
 // symmetric tangent without pivoting, then forward / diagonal / backward
-// substitution, FP64 (ProfileSPDLinDirectSolver::solve, system_of_eqn/
+// substitution (ProfileSPDLinDirectSolver::solve, system_of_eqn/
 // linearSOE/profileSPD/ProfileSPDLinDirectSolver.cpp:100-256).
 //
 // Storage: the lower triangle of the envelope (row i holds columns
 // first(i)..i, first(i) = the first column of row i in the CSR pattern) in
-// dense 32 x 32 tiles.  Tile row I keeps the tiles of columns J = I-W..I
-// (W = the widest envelope in tiles), so tile (I, J) lives at offset
+// dense 32 x 32 FP64 tiles.  Tile row I keeps the tiles of columns J =
+// I-W..I (W = the widest envelope in tiles), so tile (I, J) lives at offset
 // (I*(W+1) + I-J) * 1024, row-major inside the tile; tiles left of the
 // envelope (J < ftile[I]) stay zero and are skipped.  Right-looking LDL':
 // for every tile column J,
-//   A  the diagonal tile is factored by one block (pivots d, unit lower L);
-//   B  every tile below it becomes W_IJ = A_IJ L_JJ^-T (kept in a scratch
-//      slot) and L_IJ = W_IJ D^-1 (stored in place);
-//   C  every trailing tile pair loses W_IJ L_KJ' (one 32^3 product each).
-// The tasks (A: diagonal, B: panel tile in four row parts, C: tile pair of
-// one column; for tile (J+1, J) the four panel parts also apply a quarter
-// each of the pair (J+1, J+1)'s update, and the chain task of column J
-// factors diagonal tile J+1 -- the critical path of the factorisation) run as a dataflow: one persistent launch whose blocks take
-// tasks from a list in a fixed order -- for column J: A(J) when no column
-// updates it, the C tasks of column J-1 that reach column J+1, the panel
-// (J+1, J), the chain task, the other panels B(., J), the C tasks of column
-// J that reach column J+1, then the rest of column J-1's trailing update --
-// and
-// wait (bounded by the global timer) on per-tile counters for the tasks
-// each one depends on.  Every dependency sits earlier in the list, so the
-// look-ahead is built in: column J+1's diagonal and panels run while the
-// rest of column J's trailing update is still going.  C recovers W_IJ as
-// L_IJ D_J.  Pivot checks follow the reference: the first pivot must
-// be positive, later ones only non-zero and above minDiagTol in magnitude.
+//   A  the diagonal tile is factored (pivots d, unit lower L_JJ);
+//   B  every tile below it becomes P_IJ = A_IJ L_JJ^-T and L_IJ = P_IJ D^-1;
+//   C  every trailing tile pair loses P_IJ L_KJ'.
+// Pivot checks follow the reference: the first pivot must be positive, later
+// ones only non-zero and above minDiagTol in magnitude.
 //
-// The substitutions stream the tiles through one block: every step reads
-// one tile row (forward) or tile column (backward), accumulates it against
-// the known part of the solution and solves the diagonal tile with warp
-// shuffles.  Up to four right-hand sides share the tile loads.
+// Why the tile products run on the tensor cores.  The FP64 unit retires one
+// warp instruction per 19 cycles and SM, and one warp no more than one per
+// 64 cycles, so a 32^3 product costs 9.4 us on an SM: phase C alone would
+// take 10 us of every column of a 10 x 10 x 20 frame (165 products over 152
+// SMs).  C is therefore computed as sums of exact products: each operand row
+// is scaled by a power of two and written as nine 9-bit digits (81 bits below
+// the row's largest entry, where a double has 53), held as halves; the 45
+// digit products whose weight reaches the result run as m16n8k16 tensor-core
+// products whose float accumulators hold integers of at most 2^24 and so are
+// exact; the nine weights are added as 64-bit integers and rounded to a
+// double once.  The dropped products lie near 2^-77 of the product of the
+// rows' largest entries; the columns of both operands are scaled by powers of
+// two of sqrt(|d_k|) first, so that a row's entries (translations and
+// rotations) are of one size.  Nine digits, not seven: the entries of a
+// stiffness factor fall off by many orders along a row and FP64 keeps each to
+// its own 53 bits; with seven (63 bits, products cut at 2^-59) the solution
+// of the 10 x 10 x 20 frame lost three digits to the FP64 product, with nine
+// none.  (The idea of error-free digit products: K. Ozaki, T. Ogita, S. Oishi
+// and S. M. Rump, Numer. Algorithms 59, 2012.)
+//
+// Who runs what.  One persistent cooperative launch, a block per SM.  Tile
+// J's elimination (block `diag` J mod 3), the panel (J+1, J) (block `panel` J
+// mod 2) and that panel's update of diagonal tile J+1 (the next diag block)
+// run as a stream: the elimination publishes every column of L_JJ as it is
+// formed, the panel block solves its column with it and publishes P and L of
+// that column, the next diag block takes the column off its tile, so the next
+// tile is ready two hand-offs after the last pivot instead of after a solve
+// and a product.  These are FP64 with the operands of the plain order (an
+// explicit inverse of L_JJ would let the panels be products, but costs two
+// digits: energy norm error 7e-13 against 4e-15 on a 64 x 16 quad block).
+// The other blocks take the remaining panels (the same streamed solve), the
+// tile pairs and the substitutions' matrices from a list in look-ahead
+// order; their ninth warp draws the next task and waits for its operands
+// (bounded by the global timer) while the eight others compute.  Every
+// dependency sits earlier in the list or in the stream, and the digits live
+// in a ring of kRing tile columns (a column's slots are refilled when its
+// last pair has been applied).
 #include <cooperative_groups.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,9 +70,20 @@ namespace {
 
 constexpr int kT = 32;                 // tile edge
 constexpr int kTT = kT * kT;
-constexpr int kFactorThreads = 256;
-constexpr int kFactorSoloSmem = 120 * 1024;   // more than half an SM's shared memory
+constexpr int kComputeThreads = 256;   // the eight computing warps of a block
+constexpr int kFactorThreads = kComputeThreads + 32;
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;  // 2 s
+
+// digits of a tile operand: [kDigits][row][column] halves, then the rows'
+// exponents
+constexpr int kDigits = 9, kLowDigits = 5;   // of them in the lower word
+constexpr int kDigitBytes = kDigits * kTT * 2;
+constexpr int kOpBytes = kDigitBytes + kT * 4;
+// ring slot of a panel tile: P, then L
+constexpr int kSlotBytes = 2 * kOpBytes;
+constexpr int kRing = 8;
+constexpr int kDiagBlocks = 3, kPanelBlocks = 2;   // the stream's own blocks
+constexpr int kBadExp = 1 << 28;       // the exponent of a row with an infinity or a NaN
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -60,52 +91,43 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// (row << 5 | column) of the lower triangle of a tile, row by row
-struct LowerTable {
-  unsigned short rs[kT * (kT + 1) / 2];
-  constexpr LowerTable() : rs() {
-    int k = 0;
-    for (int r = 0; r < kT; r++)
-      for (int c = 0; c <= r; c++) rs[k++] = (unsigned short)(r * 32 + c);
-  }
-};
-__device__ const LowerTable kLowerTable{};
-#define kLowerRS (kLowerTable.rs)
-
 __device__ __forceinline__ double *tile_at(const ProfileSystem &S, int I, int o) {
   return S.L + ((size_t)I * (S.W + 1) + o) * kTT;
 }
 
-// Envelope of the CSR values into the tiles (the tiles were zeroed); rows
-// past n get a unit pivot so the padded system solves to zero there.
-__global__ void k_prof_fill(ProfileSystem S) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Before a factorisation, in one launch: every row's envelope tiles zeroed and
+// filled with the CSR values (a warp per row; rows past n get a unit pivot so
+// the padded system solves to zero there), the counters cleared, the published
+// columns and sweep values unset.
+__global__ void k_prof_prepare(ProfileSystem S, size_t ncount, size_t nsweep) {
+  const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t gthreads = (size_t)gridDim.x * blockDim.x;
+  const double none = __longlong_as_double((long long)0xFFFFFFFFFFFFFFFFull);
+  for (size_t k = gtid; k < ncount; k += gthreads) S.flags[k] = 0;
+  for (size_t k = gtid; k < 3 * (size_t)S.nt * kTT; k += gthreads) S.lstream[k] = none;
+  for (size_t k = gtid; k < nsweep; k += gthreads) S.sweep[k] = none;
   const int lane = threadIdx.x & 31;
-  const int npad = S.nt * kT;
-  if (warp >= npad) return;
-  const int i = warp, I = i / kT, r = i % kT;
-  if (i >= S.n) {
-    if (lane == 0) tile_at(S, I, 0)[r * kT + r] = 1.0;
-    return;
-  }
-  for (int k = S.rowptr[i] + lane; k < S.rowptr[i + 1]; k += 32) {
-    const int j = S.colidx[k];
-    if (j > i) continue;
-    const int J = j / kT;
-    tile_at(S, I, I - J)[r * kT + (j % kT)] = S.vals[k];
+  for (int i = (int)(gtid >> 5); i < S.nt * kT; i += (int)(gthreads >> 5)) {
+    const int I = i / kT, r = i % kT;
+    double *row = tile_at(S, I, 0) + r * kT;
+    const bool pad = i >= S.n;
+    for (int o = 0; o <= I - S.ftile[I]; o++)
+      row[(size_t)o * kTT + lane] = pad && o == 0 && lane == r ? 1.0 : 0.0;
+    __syncwarp();
+    if (pad) continue;
+    for (int k = S.rowptr[i] + lane; k < S.rowptr[i + 1]; k += 32) {
+      const int j = S.colidx[k];
+      if (j <= i) row[(size_t)(I - j / kT) * kTT + (j % kT)] = S.vals[k];
+    }
   }
 }
 
-// LDL' of diagonal tile J in shared memory (block-wide); returns false and
-// records the equation when a pivot fails the reference's checks.  Column c:
-// the column below the pivot is read and scaled by the reciprocal pivot,
-// then every trailing entry takes one FMA; the thread that finishes the
-// next pivot takes its reciprocal at once (__drcp_rn: the correctly rounded
-// 1/d, the value of the reference's 1.0/aii), so the chain of dependent
-// FP64 operations per column stays short.
-// 1/d for the elimination (xg_rcp.h); the stored reciprocal pivots are the
-// correctly rounded ones.
-__device__ __forceinline__ double elim_rcp(double d) { return chain_reciprocal(d); }
+__device__ __forceinline__ int slot_of(const ProfileSystem &S, int I, int o) {
+  return I * (S.W + 1) + o;
+}
+__device__ __forceinline__ unsigned char *dig_slot(const ProfileSystem &S, int J, int o) {
+  return S.dig + ((size_t)(J % kRing) * S.W + (o - 1)) * kSlotBytes;   // o >= 1
+}
 
 __device__ __forceinline__ void named_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
@@ -114,397 +136,564 @@ __device__ __forceinline__ void named_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
-// LDL' of the diagonal tile in sA (shared memory), as a two-stage pipeline.
-// Warp 1 carries the pivot chain: step c applies column c-1 to column c
-// (one FMA per row, the factors kept in its registers), takes the pivot's
-// reciprocal (FP64 estimate and one cubic Newton step, every lane), scales
-// the column (L below the diagonal, the unscaled column in the upper
-// triangle for the trailing update).  Warps 0, 2, 3, 4, 6 and 7 apply
-// column c to the rest of the trailing triangle (columns c+2 and beyond,
-// one FMA per entry, each thread owning up to three fixed entries) while
-// the chain goes on with column c+1; warp 5 sits out, so the chain has its
-// sub-partition's FP64 pipe to itself.  Hand-offs: named barriers 1-2
-// (chain -> trailing, by column parity) and 3-4 (trailing -> chain); the
-// chain's step c waits for the trailing update of column c-2 only.  The FMAs
-// and their operands are those of the plain right-looking order.
-constexpr int kPipeCount = 224;        // the chain warp and six trailing warps
-
-__device__ bool factor_tile(const ProfileSystem &S, int J, double (*sA)[kT + 1],
-                            volatile int *flags) {
-  double *g = tile_at(S, J, 0);
-  __shared__ double sinv[kT];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 1) {
-    double lprev = 0.0, uprev = 0.0;
-    for (int c = 0; c < kT; c++) {
-      if (c >= 2) named_sync(3 + (c & 1), kPipeCount);
-      double x = sA[lane][c];
-      if (c >= 1) {
-        const double ucc = __shfl_sync(0xffffffffu, uprev, c);
-        x = fma(-lprev, ucc, x);
-      }
-      const double d = __shfl_sync(0xffffffffu, x, c);
-      const double inv = elim_rcp(d);
-      const double l = x * inv;
-      if (lane > c) {
-        sA[lane][c] = l;
-        sA[c][lane] = x;
-      } else if (lane == c) {
-        sA[c][c] = x;
-      }
-      lprev = l;
-      uprev = x;
-      if (c <= kT - 3) named_arrive(1 + (c & 1), kPipeCount);
-    }
-  } else if (warp != 5) {
-    // this thread's entries (r, s), 2 <= s <= r < 32, column-major order
-    const int tw = (warp == 0 ? 0 : warp - 1 - (warp > 5)) * 32 + lane;
-    int ent[3];
-#pragma unroll
-    for (int u = 0; u < 3; u++) {
-      int e = tw + u * 192;
-      ent[u] = -1;
-      for (int sc = 2; sc < kT && e >= 0; sc++) {
-        if (e < kT - sc) { ent[u] = ((sc + e) << 5) | sc; break; }
-        e -= kT - sc;
-      }
-    }
-    for (int c = 0; c < kT - 2; c++) {
-      named_sync(1 + (c & 1), kPipeCount);
-#pragma unroll
-      for (int u = 0; u < 3; u++) {
-        const int e = ent[u];
-        const int r = e >> 5, sc = e & 31;
-        if (e >= 0 && sc >= c + 2) sA[r][sc] = fma(-sA[r][c], sA[c][sc], sA[r][sc]);
-      }
-      named_arrive(3 + (c & 1), kPipeCount);
-    }
-  }
-  __syncthreads();
-  if (tid < kT) sinv[tid] = __drcp_rn(sA[tid][tid]);
-  __syncwarp();
-  if (tid < kT) {
-    const int eq = J * kT + tid;
-    const double d = sA[tid][tid];
-    S.invD[eq] = sinv[tid];
-    S.piv[eq] = d;
-    // ProfileSPDLinDirectSolver.cpp:134-138 (first pivot), :189-199; the
-    // first failing pivot of the tile is reported
-    const bool fail = eq < S.n && ((eq == 0) ? !(d > 0.0)
-                                             : (d == 0.0 || fabs(d) <= S.min_diag_tol));
-    const unsigned bad = __ballot_sync(0xffffffffu, fail);
-    if (bad && tid == 0) {
-      flags[1] = J * kT + __ffs(bad) - 1;
-      __threadfence();
-      flags[0] = 3;
-    }
-  }
-  // the lower triangle (the upper one held the unscaled columns)
-  for (int k = tid; k < kTT; k += blockDim.x) {
-    const int r = k >> 5, c = k & 31;
-    g[k] = c > r ? 0.0 : sA[r][c];
-  }
-  __syncthreads();
-  return flags[0] != 3;
-}
-
-__device__ bool factor_diag(const ProfileSystem &S, int J, double (*sA)[kT + 1],
-                            volatile int *flags) {
-  const double *g = tile_at(S, J, 0);
-  for (int k = threadIdx.x; k < kTT; k += blockDim.x) sA[k >> 5][k & 31] = __ldcg(g + k);
-  __syncthreads();
-  return factor_tile(S, J, sA, flags);
-}
-
-// Phase B on rows 8q..8q+7 of tile (I = J+o, J): W = A L_JJ^-T, L = W
-// D^-1 (rows are independent, so a tile is four tasks).  A warp per row: once
-// column c of W is final (broadcast by shuffle), every later column s loses
-// W(r, c) l_sc -- no block barriers inside the sweep.
-constexpr int kPanelRows = 8;
-constexpr int kPanelParts = kT / kPanelRows;
-
-__device__ void panel_solve(const ProfileSystem &S, int J, int o, int q, double (*sA)[kT + 1],
-                            double (*sB)[kT + 1]) {
-  (void)sA;
-  const double *Ljj = tile_at(S, J, 0);
-  double *g = tile_at(S, J + o, o) + q * kPanelRows * kT;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int k = threadIdx.x; k < kTT; k += blockDim.x) sB[k >> 5][k & 31] = __ldcg(Ljj + k);
-  // warp w solves row 8q+w: lane s holds W(r, s); column c is final once
-  // the columns before it have been applied, then the later columns take it
-  double x = w < kPanelRows ? __ldcg(g + w * kT + lane) : 0.0;
-  const double inv = __ldcg(S.invD + (size_t)J * kT + lane);
-  __syncthreads();
-  if (w < kPanelRows) {
-    for (int c = 0; c < kT - 1; c++) {
-      const double wc = __shfl_sync(0xffffffffu, x, c);
-      if (lane > c) x = fma(-wc, sB[lane][c], x);
-    }
-    g[w * kT + lane] = x * inv;
-  }
-  __syncthreads();
-}
-
-// The panel of tile (J+1, J) in four row parts whose tasks, once all four
-// are written, apply a quarter each of that panel's update of diagonal tile
-// J+1 (phase C for the pair (J+1, J+1), 132 of its 528 lower entries), so
-// the chain task only factors.  The wait for the sibling parts is bounded;
-// they sit right after this task in the list, so the blocks that take them
-// never wait on this one.
-__device__ bool wait_geq_dev(const int *p, int target, volatile int *flags);
-__device__ bool panel_update_task(const ProfileSystem &S, int J, int q, double (*sA)[kT + 1],
-                                  double (*sB)[kT + 1], volatile int *flags) {
-  const int I = J + 1, tid = threadIdx.x;
-  panel_solve(S, J, 1, q, sA, sB);
-  __shared__ int ok;
-  if (tid == 0) {
-    __threadfence();
-    atomicAdd(S.done + (size_t)I * (S.W + 1) + 1, 1);
-    ok = wait_geq_dev(S.done + (size_t)I * (S.W + 1) + 1, kPanelParts, flags) &&
-         wait_geq_dev(S.upd + (size_t)I * (S.W + 1), J - S.ftile[I], flags);
-    __threadfence();
-  }
-  __syncthreads();
-  if (!ok) return false;
-  const double *gp = tile_at(S, I, 1);
-  double *gd = tile_at(S, I, 0);
-  const double *piv = S.piv + (size_t)J * kT;
-  for (int k = tid; k < kTT; k += blockDim.x) {
-    const double l = __ldcg(gp + k);
-    sB[k >> 5][k & 31] = l;
-    sA[k >> 5][k & 31] = l * __ldcg(piv + (k & 31));
-  }
-  __syncthreads();
-  constexpr int kQuarter = kT * (kT + 1) / 2 / kPanelParts;   // 132
-  for (int k = q * kQuarter + tid; k < (q + 1) * kQuarter; k += blockDim.x) {
-    const int rs = kLowerRS[k], r = rs >> 5, sc = rs & 31;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-#pragma unroll
-    for (int c = 0; c < kT; c += 4) {
-      a0 = fma(sA[r][c], sB[sc][c], a0);
-      a1 = fma(sA[r][c + 1], sB[sc][c + 1], a1);
-      a2 = fma(sA[r][c + 2], sB[sc][c + 2], a2);
-      a3 = fma(sA[r][c + 3], sB[sc][c + 3], a3);
-    }
-    gd[r * kT + sc] = __ldcg(gd + r * kT + sc) - ((a0 + a1) + (a2 + a3));
-  }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    atomicAdd(S.upd + (size_t)I * (S.W + 1), 1);
-  }
-  return true;
-}
-
-// For the substitutions, off the factorisation's critical path: W_J =
-// L_JJ^-T (rows r of W solve w L_JJ' = e_r, a warp per row as in phase B),
-// F_J = W' L_J,J-1, E_J = W' L_J,J-2, G_J = W L_J+1,J', H_J = W L_J+2,J'
-// (zero where the tile is outside the envelope), then, once row J-1's task
-// has finished, Q_J = E_J - F_J F_J-1 and R_J-1 = H_J-1 - G_J-1 G_J.  With
-// them a sweep row depends on the row two back: y_J = c3_J - F_J c_J-1 -
-// Q_J y_J-2, c_J = c3_J - E_J y_J-2 (c3_J: W' times the right-hand side
-// less rows J-3 and older), and the same backwards with G, H, R.
-__device__ void coupling_task(const ProfileSystem &S, int J, double (*sA)[kT + 1],
-                              double (*sB)[kT + 1], double (*sC)[kT + 1], volatile int *flags) {
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const size_t off = (size_t)J * kTT;
-  const double *Ljj = tile_at(S, J, 0);
-  for (int k = tid; k < kTT; k += blockDim.x) sB[k >> 5][k & 31] = __ldcg(Ljj + k);
-  __syncthreads();
-  // W = I L^-T: warp w takes rows w, w+8, w+16, w+24
-  for (int r = w; r < kT; r += blockDim.x / 32) {
-    double x = lane == r ? 1.0 : 0.0;
-    for (int c = 0; c < kT - 1; c++) {
-      const double wc = __shfl_sync(0xffffffffu, x, c);
-      if (lane > c) x = fma(-wc, sB[lane][c], x);
-    }
-    sA[r][lane] = x;
-    S.Winv[off + r * kT + lane] = x;
-  }
-  __syncthreads();
-  for (int pass = 0; pass < 4; pass++) {
-    // F = W' L_J,J-1, G = W L_J+1,J', E = W' L_J,J-2, H = W L_J+2,J'
-    const int o = pass < 2 ? 1 : 2;
-    const bool lower = (pass & 1) == 0;      // W' times a tile of row J
-    const bool has = lower ? (J >= o && S.ftile[J] <= J - o)
-                           : (J + o < S.nt && S.ftile[J + o] <= J);
-    double *out = (pass == 0 ? S.F : pass == 1 ? S.G : pass == 2 ? S.E : S.H) + off;
-    if (!has) {
-      for (int k = tid; k < kTT; k += blockDim.x) out[k] = 0.0;
-      continue;
-    }
-    const double *T = lower ? tile_at(S, J, o) : tile_at(S, J + o, o);
-    for (int k = tid; k < kTT; k += blockDim.x) sC[k >> 5][k & 31] = __ldcg(T + k);
-    __syncthreads();
-    for (int k = tid; k < kTT; k += blockDim.x) {
-      const int i = k >> 5, c = k & 31;
-      double a0 = 0.0, a1 = 0.0;
-      if (lower) {
-        for (int q = 0; q < kT; q += 2) {
-          a0 = fma(sA[q][i], sC[q][c], a0);
-          a1 = fma(sA[q + 1][i], sC[q + 1][c], a1);
-        }
-      } else {
-        for (int q = 0; q < kT; q += 2) {
-          a0 = fma(sA[i][q], sC[c][q], a0);
-          a1 = fma(sA[i][q + 1], sC[c][q + 1], a1);
-        }
-      }
-      out[k] = a0 + a1;
-    }
-    __syncthreads();
-  }
-  // Q_J and R_J-1 need row J-1's matrices (the task before this one)
-  __shared__ int ok;
-  if (tid == 0) ok = J == 0 || wait_geq_dev(S.cpl + (J - 1), 1, flags);
-  __syncthreads();
-  if (!ok) return;
-  for (int pass = 0; pass < 2; pass++) {
-    // pass 0: Q_J = E_J - F_J F_J-1;  pass 1: R_J-1 = H_J-1 - G_J-1 G_J
-    if (pass == 1 && J == 0) break;
-    const size_t oa = pass == 0 ? off : off - kTT, ob = pass == 0 ? off - kTT : off;
-    const double *A = pass == 0 ? S.F + oa : S.G + oa;
-    const double *B = pass == 0 ? S.F + ob : S.G + ob;
-    const double *C0 = pass == 0 ? S.E + off : S.H + (off - kTT);
-    double *out = pass == 0 ? S.Q + off : S.R + (off - kTT);
-    if (J == 0) {
-      for (int k = tid; k < kTT; k += blockDim.x) out[k] = __ldcg(C0 + k);
-      continue;
-    }
-    for (int k = tid; k < kTT; k += blockDim.x) {
-      sA[k >> 5][k & 31] = __ldcg(A + k);
-      sC[k >> 5][k & 31] = __ldcg(B + k);
-    }
-    __syncthreads();
-    for (int k = tid; k < kTT; k += blockDim.x) {
-      const int i = k >> 5, c = k & 31;
-      double a0 = 0.0, a1 = 0.0;
-      for (int q = 0; q < kT; q += 2) {
-        a0 = fma(sA[i][q], sC[q][c], a0);
-        a1 = fma(sA[i][q + 1], sC[q + 1][c], a1);
-      }
-      out[k] = __ldcg(C0 + k) - (a0 + a1);
-    }
-    __syncthreads();
-  }
-  // the last row's R: G_nt-1 is zero, R = H (zero as well)
-  if (J == S.nt - 1)
-    for (int k = tid; k < kTT; k += blockDim.x) S.R[off + k] = __ldcg(S.H + off + k);
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    atomicExch(S.cpl + J, 1);
-  }
-}
-
-// Phase C on pair (I = J+a, K = J+b), b <= a: A_IK -= (L_IJ D_J) L_KJ'.
-__device__ void pair_update(const ProfileSystem &S, int J, int a, int b, double (*sA)[kT + 1],
-                            double (*sB)[kT + 1]) {
-  const double *li = tile_at(S, J + a, a);
-  const double *lk = tile_at(S, J + b, b);
-  const double *piv = S.piv + (size_t)J * kT;
-  for (int k = threadIdx.x; k < kTT; k += blockDim.x) {
-    sA[k / kT][k % kT] = __ldcg(li + k) * __ldcg(piv + k % kT);
-    sB[k / kT][k % kT] = __ldcg(lk + k);
-  }
-  __syncthreads();
-  double *out = tile_at(S, J + a, a - b);
-  if (a == b) {
-    // a diagonal tile: its lower triangle only (528 entries, packed table)
-    for (int k = threadIdx.x; k < kT * (kT + 1) / 2; k += blockDim.x) {
-      const int rs = kLowerRS[k], r = rs >> 5, s = rs & 31;
-      double acc = 0.0;
-#pragma unroll 8
-      for (int c = 0; c < kT; c++) acc += sA[r][c] * sB[s][c];
-      out[r * kT + s] = __ldcg(out + r * kT + s) - acc;
-    }
-  } else {
-    for (int k = threadIdx.x; k < kTT; k += blockDim.x) {
-      const int r = k / kT, s = k % kT;
-      double acc = 0.0;
-#pragma unroll 8
-      for (int c = 0; c < kT; c++) acc += sA[r][c] * sB[s][c];
-      out[k] = __ldcg(out + k) - acc;
-    }
-  }
-  __syncthreads();
-}
-
-__device__ bool wait_geq(const int *p, int target, volatile int *flags);
-__device__ bool wait_geq_dev(const int *p, int target, volatile int *flags) {
-  return wait_geq(p, target, flags);
-}
-
-__device__ __forceinline__ int slot_of(const ProfileSystem &S, int I, int o) {
-  return I * (S.W + 1) + o;
-}
-
-// Column J's critical chain: once the four panel-part tasks of tile
-// (J+1, J) have applied their quarters of its update of diagonal tile J+1,
-// that tile's LDL' in shared memory.
-__device__ bool chain_task(const ProfileSystem &S, int J, double (*sC)[kT + 1],
-                           volatile int *flags) {
-  return factor_diag(S, J + 1, sC, flags);
-}
-
-// Wait until *p >= target (thread 0 of a block); false on a raised error
-// flag or after kBarrierTimeoutNs (flags[0] = 2).
-__device__ bool wait_geq(const int *p, int target, volatile int *flags) {
+// Wait until *p >= target (one thread); false on a raised error flag or after
+// kBarrierTimeoutNs (flags[0] = 2).
+__device__ __noinline__ bool wait_slow(const int *p, int target, volatile int *flags) {
   const volatile int *vp = p;
-  if (*vp >= target) return true;
   const unsigned long long t0 = global_ns();
-  while (*vp < target) {
+  for (;;) {
+    for (int k = 0; k < 32; k++)
+      if (*vp >= target) return true;
     if (flags[0] != 0) return false;
     if (global_ns() - t0 > kBarrierTimeoutNs) {
       flags[0] = 2;
       return false;
     }
-    __nanosleep(20);
   }
-  return true;
+}
+__device__ __forceinline__ bool wait_geq(const int *p, int target, volatile int *flags) {
+  return *(const volatile int *)p >= target || wait_slow(p, target, flags);
 }
 
-// Dependencies of a task: every update of its tile from earlier columns
-// (the count of columns J' < J both tile rows reach), and the diagonal /
-// panel tiles it reads.
+// Published values: a scratch vector is filled with kUnset beforehand (a NaN
+// pattern that no arithmetic result is stored as) and a consumer polls
+// exactly the values it reads, so a value and its arrival are one word.
+constexpr unsigned long long kUnset = 0xFFFFFFFFFFFFFFFFull;   // byte fill 0xFF
+
+__device__ __forceinline__ double ld_relaxed(const double *p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ bool unset(double v) {
+  return (unsigned long long)__double_as_longlong(v) == kUnset;
+}
+
+// *p once its producer has published it; 0 after a failed wait (flags[0]
+// is then nonzero and the host reports the solve as failed).  await_slow is
+// for the sweeps, where 64 blocks of threads poll and a look at the flag and
+// the clock between two loads keeps them from crowding the L2 (981 against
+// 1,108 us a backward sweep of 454 tile rows); await_column for the few warps
+// that follow the factorisation's stream.
+__device__ __forceinline__ double await_slow(const double *p, volatile int *flags) {
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+    const double v = ld_relaxed(p);
+    if (!unset(v)) return v;
+    if (flags[0] != 0) return 0.0;
+    if (global_ns() - t0 > kBarrierTimeoutNs) {
+      flags[0] = 2;
+      return 0.0;
+    }
+  }
+}
+__device__ __forceinline__ double await_column(const double *p, volatile int *flags) {
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int k = 0; k < 32; k++) {
+      const double v = ld_relaxed(p);
+      if (!unset(v)) return v;
+    }
+    if (flags[0] != 0) return 0.0;
+    if (global_ns() - t0 > kBarrierTimeoutNs) {
+      flags[0] = 2;
+      return 0.0;
+    }
+  }
+}
+
+// p[0], p[8], p[16], p[24] (the four loads in flight together)
+__device__ __forceinline__ void await4(const double *p, double v[4], volatile int *flags) {
+#pragma unroll
+  for (int m = 0; m < 4; m++) v[m] = ld_relaxed(p + 8 * m);
+#pragma unroll
+  for (int m = 0; m < 4; m++)
+    if (unset(v[m])) v[m] = await_slow(p + 8 * m, flags);
+}
+
+__device__ __forceinline__ void publish(double *p, double v) {
+  if (unset(v)) v = __longlong_as_double(0x7FF8000000000000ll);   // keep a NaN a NaN
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+// the eight computing warps
+__device__ __forceinline__ void csync() { named_sync(9, kComputeThreads); }
+
+// floor(log2(|v|) / 2): the power of two that brings sqrt(|v|) near 1
+__device__ __forceinline__ int half_exp(double v) {
+  const int be = (__double2hiint(v) >> 20) & 0x7ff;
+  return (be == 0 || be == 0x7ff) ? 0 : (be - 1023) >> 1;
+}
+
+// Four consecutive entries of row r (columns 4q .. 4q+3, the eight threads
+// of a row adjacent lanes of a warp), scaled by 2^-cs, as digits of |v|, v =
+// x 2^(79-E), |x 2^-cs| < 2^E over the row, in two words of four and five
+// digits: |v| plus 256 in every digit place has unsigned 9-bit fields, each
+// 256 above its signed digit; a field in a half's mantissa under the exponent
+// of 1024 is 1024 + field, 1280 less is the digit, and v's sign goes onto
+// every digit.
+__device__ __forceinline__ void slice_row4(const double (&x)[4], const int (&cs)[4], int r, int q,
+                                           unsigned char *dst) {
+  int e[4], em = -(1 << 20);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int be = (__double2hiint(x[i]) >> 20) & 0x7ff;
+    e[i] = be == 0 ? -(1 << 20) : be == 0x7ff ? kBadExp : be - cs[i];
+    em = max(em, e[i]);
+  }
+  em = max(em, __shfl_xor_sync(0xffffffffu, em, 1));
+  em = max(em, __shfl_xor_sync(0xffffffffu, em, 2));
+  em = max(em, __shfl_xor_sync(0xffffffffu, em, 4));
+  const bool bad = em >= kBadExp - (1 << 16);
+  constexpr int kLowBits = 9 * kLowDigits;
+  constexpr unsigned long long kLowMask = (1ull << kLowBits) - 1;
+  constexpr unsigned long long kBiasLow = 0x1008040201ull << 8, kBiasHigh = 0x8040201ull << 8;
+  unsigned long long uh[4], ul[4];
+  unsigned sg[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int hi = __double2hiint(x[i]), lo = __double2loint(x[i]);
+    unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)lo;
+    int sh = 26 - (em - e[i]);
+    if (bad || sh <= -54 || e[i] <= -(1 << 19)) m = 0;
+    if (sh < 0) {
+      sh = max(sh, -63);
+      m = (m + (1ull << (-sh - 1))) >> -sh;
+      sh = 0;
+    }
+    ul[i] = ((m << sh) & kLowMask) + kBiasLow;
+    uh[i] = (m >> (kLowBits - sh)) + kBiasHigh + (ul[i] >> kLowBits);
+    sg[i] = ((unsigned)hi >> 16) & 0x8000u;
+  }
+  const size_t at = (size_t)(r * kT + 4 * q) * 2;
+  const __half2 k1280 = __halves2half2(__ushort_as_half(0x6500), __ushort_as_half(0x6500));
+#pragma unroll
+  for (int d = 0; d < kDigits; d++) {
+    constexpr int kHigh = kDigits - kLowDigits;
+    const int s = 9 * ((d < kHigh ? kHigh : kDigits) - 1 - d);
+    unsigned f[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) f[i] = (unsigned)((d < kHigh ? uh[i] : ul[i]) >> s) & 511u;
+    unsigned w0 = f[0] | (f[1] << 16) | 0x64006400u, w1 = f[2] | (f[3] << 16) | 0x64006400u;
+    const __half2 h0 = __hsub2(*reinterpret_cast<__half2 *>(&w0), k1280);
+    const __half2 h1 = __hsub2(*reinterpret_cast<__half2 *>(&w1), k1280);
+    w0 = *reinterpret_cast<const unsigned *>(&h0) ^ (sg[0] | (sg[1] << 16));
+    w1 = *reinterpret_cast<const unsigned *>(&h1) ^ (sg[2] | (sg[3] << 16));
+    *reinterpret_cast<uint2 *>(dst + d * kTT * 2 + at) = make_uint2(w0, w1);
+  }
+  if (q == 0)
+    *reinterpret_cast<int *>(dst + kDigitBytes + 4 * r) =
+        bad ? kBadExp : em <= -(1 << 16) ? 0 : em - 1022;
+}
+
+__device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
+                                         unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// (hi 2^36 + lo) 2^sc rounded to a double (to nearest, ties up); |hi| < 2^62,
+// |lo| < 2^63
+__device__ __forceinline__ double fixed_to_double(long long hi, long long lo, int sc) {
+  if (sc >= kBadExp / 2) return __longlong_as_double(0x7ff8000000000000ll);
+  hi += lo >> 36;
+  unsigned long long rem = (unsigned long long)lo & 0xfffffffffull;
+  const bool neg = hi < 0;
+  if (neg) {
+    hi = rem ? ~hi : -hi;
+    rem = (0x1000000000ull - rem) & 0xfffffffffull;
+  }
+  const int k = min(__clzll(hi), 36);
+  const unsigned long long m = ((unsigned long long)hi << k) | (rem >> (36 - k));
+  if (m == 0) return 0.0;
+  const int lz = __clzll((long long)m);
+  const unsigned long long n = m << lz;
+  const int be = 1023 + 63 - lz + sc + 36 - k;
+  unsigned long long bits = ((unsigned long long)(be - 1) << 52) + (n >> 11) + ((n >> 10) & 1);
+  if (be <= 0) bits = 0;
+  if (be >= 2047) bits = 0x7ff0000000000000ull;
+  if (neg) bits |= 0x8000000000000000ull;
+  return __longlong_as_double((long long)bits);
+}
+
+// Rows m0..m0+15 against rows n0..n0+7 of two operands: out = sums over the
+// 32 columns, in the m16n8 accumulator layout (rows m0 + lane/4 and 8 more,
+// columns n0 + 2 (lane % 4) and the next).  A lane takes columns 8 (lane %
+// 4) .. +7 of its rows as its share of the contraction, the same for both
+// operands, so a digit of a row is one 16-byte load (the operands are
+// written during this launch: read through the L2).
+__device__ __forceinline__ uint4 frag(const unsigned char *op, int d, int row, int t) {
+  return __ldcg(reinterpret_cast<const uint4 *>(op) + (d * kT + row) * 4 + t);
+}
+__device__ __forceinline__ int row_exp(const unsigned char *op, int row) {
+  return __ldcg(reinterpret_cast<const int *>(op + kDigitBytes) + row);
+}
+__device__ __forceinline__ void tile_product(const unsigned char *A, const unsigned char *B, int m0,
+                                             int n0, int lane, double (&out)[4]) {
+  const int g = lane >> 2, t = lane & 3;
+  uint4 a0[kDigits], a1[kDigits], b[kDigits];
+#pragma unroll
+  for (int d = 0; d < kDigits; d++) {
+    a0[d] = frag(A, d, m0 + g, t);
+    a1[d] = frag(A, d, m0 + 8 + g, t);
+    b[d] = frag(B, d, n0 + g, t);
+  }
+  const int ea0 = row_exp(A, m0 + g), ea1 = row_exp(A, m0 + 8 + g);
+  const int eb0 = row_exp(B, n0 + 2 * t), eb1 = row_exp(B, n0 + 2 * t + 1);
+  float acc[kDigits][4];
+#pragma unroll
+  for (int u = 0; u < kDigits; u++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) acc[u][k] = 0.f;
+#pragma unroll
+  for (int i = 0; i < kDigits; i++) {
+#pragma unroll
+    for (int j = 0; j < kDigits - i; j++)
+      mma16816(acc[i + j], a0[i].x, a1[i].x, a0[i].y, a1[i].y, b[j].x, b[j].y);
+#pragma unroll
+    for (int j = 0; j < kDigits - i; j++)
+      mma16816(acc[i + j], a0[i].z, a1[i].z, a0[i].w, a1[i].w, b[j].z, b[j].w);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    // weights 2^36 .. 1 of two words; the value is (hi 2^36 + lo) 2^(Ea+Eb-86)
+    long long hi = 0, lo = 0;
+#pragma unroll
+    for (int u = 0; u < kDigits; u++) {
+      const long long v = __float2int_rn(acc[u][k]);
+      if (u < kDigits - 4) hi += v << (9 * (kDigits - 5 - u));
+      else lo += v << (9 * (kDigits - 1 - u));
+    }
+    out[k] = fixed_to_double(hi, lo, (k < 2 ? ea0 : ea1) + ((k & 1) ? eb1 : eb0) - 86);
+  }
+}
+
+struct FactorSmem {
+  double A[kT][kT + 1];          // the tile at hand, by rows
+  double W[kT][kT + 1];          // columns: a panel's P, a diagonal tile's unscaled columns
+  double L[kT][kT + 1];          // and their L
+  double inv[kT];                // reciprocal pivots of the panel's column
+  double Lc[2][kT];              // the published column being applied
+  int4 task[2];
+  int fail;
+};
+// more than half an SM's shared memory: one block per SM
+constexpr int kFactorSmem = 120 * 1024;
+static_assert(sizeof(FactorSmem) <= kFactorSmem, "");
+
+__device__ __forceinline__ void load4(const double *g, double (&x)[4]) {
+  const double2 a = __ldcg(reinterpret_cast<const double2 *>(g));
+  const double2 b = __ldcg(reinterpret_cast<const double2 *>(g) + 1);
+  x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+}
+
+// LDL' of the diagonal tile in sm.A, as a two-stage pipeline, its columns of
+// L published to st ([column][row], the reciprocal pivot on the diagonal) as
+// they are formed; sm.L keeps them by columns (the pivot on the diagonal),
+// sm.W the unscaled columns.  Warp 0 carries the pivot chain: with column c
+// final it takes the pivot's reciprocal (xg_rcp.h), scales the column,
+// applies it to column c+1 (one FMA per row) and, in the shadow of that FMA,
+// writes column c out for warps 1-6, which apply it to columns c+3 and beyond
+// (one FMA per entry, each thread holding up to three fixed entries).  The
+// raw column c+1 with column c-1 applied, and its factor, are formed in the
+// shadow of the reciprocal, so the trailing warps have two columns' time.
+// An FP64 result reaches another FP64 operation after 64 cycles and any other
+// unit after 90; a divergent branch on the chain costs 50-100 cycles, so it
+// has none: every lane writes, also the rows above the diagonal that nobody
+// reads, and the reciprocal's range is looked at behind the FMA.  520 cycles
+// a column; 815 with the column written out under branches before the FMA and
+// the reciprocal in FP64.  Hand-offs: named barriers 1-2 (chain -> trailing,
+// by column parity) and 3-4 (trailing -> chain).  The FMAs and their operands
+// are those of the plain right-looking order.
+constexpr int kPipeCount = 7 * 32;      // the chain warp and six trailing warps
+struct TrailEntries { int rw[3], sc[3]; };
+// this thread's entries (r, s), 3 <= s <= r < 32, column-major order
+__device__ __forceinline__ TrailEntries trail_entries(int warp, int lane) {
+  TrailEntries t;
+#pragma unroll
+  for (int u = 0; u < 3; u++) {
+    int e = (warp - 1) * 32 + lane + u * 192;
+    t.rw[u] = t.sc[u] = -1;
+    if (warp < 1 || warp > 6) continue;
+    for (int k = 3; k < kT; k++) {
+      if (e < kT - k) { t.rw[u] = k + e; t.sc[u] = k; break; }
+      e -= kT - k;
+    }
+  }
+  return t;
+}
+__device__ void eliminate_tile(FactorSmem &sm, int warp, int lane, const TrailEntries &te,
+                               double *st) {
+  if (warp == 0) {
+    double x = sm.A[lane][0], lp = 0.0, up = 0.0;
+#pragma unroll 1
+    for (int c = 0; c < kT; c++) {
+      const double d = __shfl_sync(0xffffffffu, x, c);
+      double raw = 0.0, ucc = 0.0;
+      if (c < kT - 1) {
+        if (c >= 2) named_sync(3 + (c & 1), kPipeCount);
+        raw = sm.A[lane][c + 1];
+        ucc = __shfl_sync(0xffffffffu, x, c + 1);
+        const double up1 = __shfl_sync(0xffffffffu, up, c + 1);
+        if (c >= 1) raw = fma(-lp, up1, raw);
+      }
+      double inv = wide_reciprocal(d);
+      double l = x * inv;
+      double xn = fma(-l, ucc, raw);
+      if (reciprocal_out_of_range(d)) {
+        inv = __drcp_rn(d);
+        l = x * inv;
+        xn = fma(-l, ucc, raw);
+      }
+      sm.L[c][lane] = lane == c ? x : l;
+      sm.W[c][lane] = x;
+      if (c <= kT - 4) named_arrive(1 + (c & 1), kPipeCount);
+      publish(st + c * kT + lane, lane == c ? inv : l);
+      lp = l;
+      up = x;
+      x = xn;
+    }
+  } else if (warp <= 6) {
+    double m[3];
+#pragma unroll
+    for (int u = 0; u < 3; u++) m[u] = te.rw[u] >= 0 ? sm.A[te.rw[u]][te.sc[u]] : 0.0;
+    for (int c = 0; c < kT - 3; c++) {
+      named_sync(1 + (c & 1), kPipeCount);
+#pragma unroll
+      for (int u = 0; u < 3; u++) {
+        if (te.sc[u] >= c + 3) {
+          m[u] = fma(-sm.L[c][te.rw[u]], sm.W[c][te.sc[u]], m[u]);
+          if (te.sc[u] == c + 3) sm.A[te.rw[u]][c + 3] = m[u];
+        }
+      }
+      named_arrive(3 + (c & 1), kPipeCount);
+    }
+  }
+}
+
+// Phase B on tile (I, J): P L_JJ' = A, L = P D^-1, column by column as L_JJ
+// is published.  Lane = row; warp w of the eight computing ones holds columns
+// w, w+8, w+16, w+24 in registers, so that a column's FMAs fill whole warps
+// (496 in all: 9,400 cycles of the FP64 unit, below the elimination's own
+// time); the warp whose column is final hands it to the others through shared
+// memory.  The ninth warp polls the published columns (panel_poll), a column
+// ahead of the others; one barrier a column.  With wl, P and L of each column
+// are published for the block that holds diagonal tile I.  Afterwards L goes
+// to the tile and both, as digits, to the ring slot.
+__device__ void panel_poll(const ProfileSystem &S, FactorSmem &sm, int J, int lane,
+                           volatile int *flags) {
+  const double *st = S.lstream + (size_t)J * kTT;
+  double v = ld_relaxed(st + lane);
+  for (int c = 0; c < kT; c++) {
+    if (lane >= c) {
+      if (unset(v)) v = await_column(st + c * kT + lane, flags);
+      sm.Lc[c & 1][lane] = v;
+      if (lane > c) v = ld_relaxed(st + (c + 1) * kT + lane);
+    }
+    __syncwarp();
+    named_sync(10, kFactorThreads);
+  }
+}
+__device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J, int tid,
+                           double *wl) {
+  const int r = tid >> 3, q = tid & 7, o = I - J, w = tid >> 5, lane = tid & 31;
+  double *tile = tile_at(S, I, o) + r * kT + 4 * q;
+  double x[4];
+  load4(tile, x);
+#pragma unroll
+  for (int i = 0; i < 4; i++) sm.A[r][4 * q + i] = x[i];
+  csync();
+#pragma unroll
+  for (int j = 0; j < 4; j++) x[j] = sm.A[lane][8 * j + w];
+  if (w == 0) {
+    sm.W[0][lane] = x[0];
+    if (wl) publish(wl + lane, x[0]);
+  }
+#pragma unroll
+  for (int jc = 0; jc < 4; jc++) {
+    for (int c8 = 0; c8 < 8; c8++) {
+      const int c = 8 * jc + c8;
+      named_sync(10, kFactorThreads);
+      const double wc = sm.W[c][lane];
+      const double *lc = sm.Lc[c & 1];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int s = 8 * j + w;
+        if (j >= jc && s > c) {
+          x[j] = fma(-wc, lc[s], x[j]);
+          if (s == c + 1) {
+            sm.W[s][lane] = x[j];
+            if (wl) publish(wl + s * 2 * kT + lane, x[j]);
+          }
+        }
+      }
+      if (w == c8) {      // column c is this warp's: scale it
+        const double inv = lc[c], v = x[jc] * inv;
+        sm.L[c][lane] = v;
+        if (lane == 0) sm.inv[c] = inv;
+        if (wl) publish(wl + c * 2 * kT + kT + lane, v);
+      }
+    }
+  }
+  csync();
+  double p[4], l[4];
+  int t[4], nt[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    p[i] = sm.W[4 * q + i][r];
+    l[i] = sm.L[4 * q + i][r];
+    nt[i] = half_exp(sm.inv[4 * q + i]);
+    t[i] = -nt[i];
+  }
+  reinterpret_cast<double2 *>(tile)[0] = make_double2(l[0], l[1]);
+  reinterpret_cast<double2 *>(tile)[1] = make_double2(l[2], l[3]);
+  unsigned char *slot = dig_slot(S, J, o);
+  slice_row4(p, t, r, q, slot);
+  slice_row4(l, nt, r, q, slot + kOpBytes);
+}
+
+// Phase C on pair (I = J+a, K = J+b), b <= a: A_IK -= P_IJ L_KJ'.  On a
+// diagonal tile the blocks above the diagonal are left out.
+__device__ void pair_task(const ProfileSystem &S, int J, int a, int b, int tid) {
+  const int w = tid >> 5, lane = tid & 31, m0 = (w >> 2) * 16, n0 = (w & 3) * 8;
+  if (a == b && n0 >= m0 + 16) return;
+  const int g = lane >> 2, t = lane & 3;
+  double2 *c0 = reinterpret_cast<double2 *>(tile_at(S, J + a, a - b) + (m0 + g) * kT + n0 + 2 * t);
+  double2 *c1 = c0 + 4 * kT;
+  const double2 v0 = __ldcg(c0), v1 = __ldcg(c1);
+  double out[4];
+  tile_product(dig_slot(S, J, a), dig_slot(S, J, b) + kOpBytes, m0, n0, lane, out);
+  *c0 = make_double2(v0.x - out[0], v0.y - out[1]);
+  *c1 = make_double2(v1.x - out[2], v1.y - out[3]);
+}
+
+// W_J = L_JJ^-T for the substitutions: rows r of W solve w L_JJ' = e_r, a
+// warp per row
+__device__ void inverse_task(const ProfileSystem &S, FactorSmem &sm, int J, int tid) {
+  const int w = tid >> 5, lane = tid & 31;
+  const double *Ljj = tile_at(S, J, 0);
+  for (int k = tid; k < kTT; k += kComputeThreads) sm.A[k >> 5][k & 31] = __ldcg(Ljj + k);
+  csync();
+  for (int r = w; r < kT; r += kComputeThreads / 32) {
+    double x = lane == r ? 1.0 : 0.0;
+    for (int c = r; c < kT - 1; c++) {
+      const double wc = __shfl_sync(0xffffffffu, x, c);
+      if (lane > c) x = fma(-wc, sm.A[lane][c], x);
+    }
+    S.Winv[(size_t)J * kTT + r * kT + lane] = x;
+  }
+}
+
+// For the substitutions, off the chain, with W_J = L_JJ^-T: pass 0
+// F_J = W' L_J,J-1, 1 G_J = W L_J+1,J', 2 E_J = W' L_J,J-2, 3 H_J = W
+// L_J+2,J' (zero where the tile is outside the envelope), a task each; then
+// Q_J = E_J - F_J F_J-1 and R_J = H_J - G_J G_J+1.  With them a sweep row
+// depends on the row two back: y_J = c3_J - F_J c_J-1 - Q_J y_J-2, c_J =
+// c3_J - E_J y_J-2 (c3_J: W' times the right-hand side less rows J-3 and
+// older), and the same backwards with G, H, R.
+__device__ __forceinline__ bool coupling_tile(const ProfileSystem &S, int J, int pass, int *I,
+                                              int *o) {
+  const bool lower = (pass & 1) == 0;      // W' times a tile of row J
+  *o = pass < 2 ? 1 : 2;
+  *I = lower ? J : J + *o;
+  return lower ? (J >= *o && S.ftile[J] <= J - *o) : (J + *o < S.nt && S.ftile[J + *o] <= J);
+}
+__device__ void coupling_task(const ProfileSystem &S, FactorSmem &sm, int J, int pass, int tid) {
+  int I, o;
+  const bool has = coupling_tile(S, J, pass, &I, &o), lower = (pass & 1) == 0;
+  const size_t off = (size_t)J * kTT;
+  double *out = (pass == 0 ? S.F : pass == 1 ? S.G : pass == 2 ? S.E : S.H) + off;
+  if (!has) {
+    for (int k = tid; k < kTT; k += kComputeThreads) out[k] = 0.0;
+    return;
+  }
+  const double *T = tile_at(S, I, o);
+  for (int k = tid; k < kTT; k += kComputeThreads) {
+    sm.A[k >> 5][k & 31] = __ldcg(S.Winv + off + k);
+    sm.W[k >> 5][k & 31] = __ldcg(T + k);
+  }
+  csync();
+  for (int k = tid; k < kTT; k += kComputeThreads) {
+    const int i = k >> 5, c = k & 31;
+    double a0 = 0.0, a1 = 0.0;
+    if (lower) {
+      for (int q = 0; q < kT; q += 2) {
+        a0 = fma(sm.A[q][i], sm.W[q][c], a0);
+        a1 = fma(sm.A[q + 1][i], sm.W[q + 1][c], a1);
+      }
+    } else {
+      for (int q = 0; q < kT; q += 2) {
+        a0 = fma(sm.A[i][q], sm.W[c][q], a0);
+        a1 = fma(sm.A[i][q + 1], sm.W[c][q + 1], a1);
+      }
+    }
+    out[k] = a0 + a1;
+  }
+}
+// which 0: Q_J, 1: R_J
+__device__ void second_coupling_task(const ProfileSystem &S, FactorSmem &sm, int J, int which,
+                                     int tid) {
+  const size_t off = (size_t)J * kTT;
+  const double *C0 = (which == 0 ? S.E : S.H) + off;
+  double *out = (which == 0 ? S.Q : S.R) + off;
+  if (which == 0 ? J == 0 : J == S.nt - 1) {
+    for (int k = tid; k < kTT; k += kComputeThreads) out[k] = __ldcg(C0 + k);
+    return;
+  }
+  const double *A = (which == 0 ? S.F : S.G) + off;
+  const double *B = which == 0 ? A - kTT : A + kTT;
+  for (int k = tid; k < kTT; k += kComputeThreads) {
+    sm.A[k >> 5][k & 31] = __ldcg(A + k);
+    sm.W[k >> 5][k & 31] = __ldcg(B + k);
+  }
+  csync();
+  for (int k = tid; k < kTT; k += kComputeThreads) {
+    const int i = k >> 5, c = k & 31;
+    double a0 = 0.0, a1 = 0.0;
+    for (int q = 0; q < kT; q += 2) {
+      a0 = fma(sm.A[i][q], sm.W[q][c], a0);
+      a1 = fma(sm.A[i][q + 1], sm.W[q + 1][c], a1);
+    }
+    out[k] = __ldcg(C0 + k) - (a0 + a1);
+  }
+}
+
+// Dependencies of a list task (type, I, K, J): every update of its tile from
+// earlier columns (the count of columns J' < J both tile rows reach), and the
+// diagonal / panel tiles it reads.
+enum { kPanel = 1, kPair = 2, kInverse = 5, kCouple = 6, kForward = 7, kCouple2 = 8 };
 __device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
   const int type = t.x, I = t.y, K = t.z, J = t.w;
-  if (type == 0)
-    return wait_geq(S.upd + slot_of(S, J, 0), J - S.ftile[J], flags);
-  if (type == 4)
-    return wait_geq(S.upd + slot_of(S, I, 0), J - S.ftile[I] + kPanelParts, flags);
-  if (type == 5)
-    return wait_geq(S.done + slot_of(S, J, 0), 1, flags) &&
-           wait_geq(S.upd + slot_of(S, I, 1), J - max(S.ftile[I], S.ftile[J]), flags);
-  if (type == 6) {
-    if (!wait_geq(S.done + slot_of(S, J, 0), 1, flags)) return false;
-    for (int o = 1; o <= 2; o++) {
-      if (J >= o && S.ftile[J] <= J - o &&
-          !wait_geq(S.done + slot_of(S, J, o), kPanelParts, flags))
-        return false;
-      if (J + o < S.nt && S.ftile[J + o] <= J &&
-          !wait_geq(S.done + slot_of(S, J + o, o), kPanelParts, flags))
-        return false;
-    }
-    return true;
-  }
-  if (type == 7) {
-    // row J's forward step: its coupling matrices and the panel tiles of
-    // the row further left (the y values of the rows before it are polled
-    // inside the step)
-    if (S.fwd_nrhs == 0) return true;
-    if (!wait_geq(S.cpl + J, 1, flags)) return false;
-    const int ohi = min(S.W, J - S.ftile[J]);
-    for (int o = 3; o <= ohi; o++)
-      if (!wait_geq(S.done + slot_of(S, J, o), kPanelParts, flags)) return false;
-    return true;
-  }
-  if (type == 1)
-    return wait_geq(S.done + slot_of(S, J, 0), 1, flags) &&
+  if (type == kPanel)     // the columns of L_JJ are polled inside the task
+    return (J < kRing || wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags)) &&
            wait_geq(S.upd + slot_of(S, I, I - J), J - max(S.ftile[I], S.ftile[J]), flags);
-  return wait_geq(S.done + slot_of(S, I, I - J), kPanelParts, flags) &&
-         wait_geq(S.done + slot_of(S, K, K - J), kPanelParts, flags) &&
-         wait_geq(S.upd + slot_of(S, I, I - K), J - max(S.ftile[I], S.ftile[K]), flags);
+  if (type == kPair)
+    return wait_geq(S.done + slot_of(S, I, I - J), 1, flags) &&
+           wait_geq(S.done + slot_of(S, K, K - J), 1, flags) &&
+           wait_geq(S.upd + slot_of(S, I, I - K), J - max(S.ftile[I], S.ftile[K]), flags);
+  if (type == kInverse) return wait_geq(S.done + slot_of(S, J, 0), 1, flags);
+  if (type == kCouple) {
+    int Ic, o;
+    if (!wait_geq(S.cplw + J, 1, flags)) return false;
+    return !coupling_tile(S, J, K, &Ic, &o) || wait_geq(S.done + slot_of(S, Ic, o), 1, flags);
+  }
+  if (type == kCouple2) {
+    const int O = K == 0 ? J - 1 : J + 1;    // the neighbour's F or G
+    return wait_geq(S.cpl + J, 4, flags) && (O < 0 || O >= S.nt || wait_geq(S.cpl + O, 4, flags));
+  }
+  // row J's forward step: its coupling matrices and the panel tiles of the
+  // row further left (the y values of the rows before it are polled inside
+  // the step)
+  if (S.fwd_nrhs == 0) return true;
+  if (!wait_geq(S.cplq + J, 1, flags)) return false;
+  const int ohi = min(S.W, J - S.ftile[J]);
+  for (int o = 3; o <= ohi; o++)
+    if (!wait_geq(S.done + slot_of(S, J, o), 1, flags)) return false;
+  return true;
 }
 
 // Pipelined substitutions on kPipeBlocks co-resident blocks (cooperative
@@ -523,46 +712,9 @@ __device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
 // values it reads.  Waits are bounded by the global timer.
 constexpr int kPipeBlocks = 64;
 constexpr int kPipeThreads = 256;
-constexpr unsigned long long kUnset = 0xFFFFFFFFFFFFFFFFull;   // byte fill 0xFF
-
-__device__ __forceinline__ double ld_relaxed(const double *p) {
-  double v;
-  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
-// *p once its producer has published it; 0 after a failed wait (flags[0]
-// is then nonzero and the host reports the solve as failed)
-__device__ __forceinline__ double await_value(const double *p, volatile int *flags) {
-  double v = ld_relaxed(p);
-  if ((unsigned long long)__double_as_longlong(v) != kUnset) return v;
-  const unsigned long long t0 = global_ns();
-  for (;;) {
-    v = ld_relaxed(p);
-    if ((unsigned long long)__double_as_longlong(v) != kUnset) return v;
-    if (flags[0] != 0) return 0.0;
-    if (global_ns() - t0 > kBarrierTimeoutNs) {
-      flags[0] = 2;
-      return 0.0;
-    }
-  }
-}
-
-// p[0], p[8], p[16], p[24] (the four loads in flight together)
-__device__ __forceinline__ void await4(const double *p, double v[4], volatile int *flags) {
-  bool ready = true;
-#pragma unroll
-  for (int m = 0; m < 4; m++) v[m] = ld_relaxed(p + 8 * m);
-#pragma unroll
-  for (int m = 0; m < 4; m++) ready &= (unsigned long long)__double_as_longlong(v[m]) != kUnset;
-  if (!ready)
-    for (int m = 0; m < 4; m++) v[m] = await_value(p + 8 * m, flags);
-}
-
-__device__ __forceinline__ void publish(double *p, double v) {
-  if ((unsigned long long)__double_as_longlong(v) == kUnset)
-    v = __longlong_as_double(0x7FF8000000000000ll);   // keep a NaN a NaN
-  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+// right-hand side q, zero past the last equation
+__device__ __forceinline__ double rhs_at(const ProfileSystem &S, int q, int i) {
+  return i < S.n ? __ldcg(S.b[q] + i) : 0.0;
 }
 
 // Forward substitution of tile row J for the right-hand sides given to the
@@ -612,7 +764,7 @@ __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
   }
   for (int q = 0; q < nrhs; q++) {
     const double v = group_sum(acc[q]);
-    if (g == 0) rb[q][r] = __ldcg(S.fwd_x + (size_t)q * S.fwd_ldx + J * kT + r) - v;
+    if (g == 0) rb[q][r] = rhs_at(S, q, J * kT + r) - v;
   }
   const double *Wt = S.Winv + (size_t)J * kTT;
   double wv[4];
@@ -623,7 +775,7 @@ __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
   row_of(S.F + off, fv);
   row_of(S.Q + off, qv);
   row_of(S.E + off, ev);
-  __syncthreads();
+  csync();
   const bool hasF = J >= 1 && S.ftile[J] <= J - 1;
   for (int q = 0; q < nrhs; q++) {
     double c3 = 0.0;
@@ -641,154 +793,226 @@ __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
   return flags[0] == 0;
 }
 
-__global__ void __launch_bounds__(kFactorThreads) k_prof_factor(ProfileSystem S) {
-  __shared__ double sA[kT][kT + 1], sB[kT][kT + 1], sC[kT][kT + 1];
-  __shared__ int task, ok;
-  volatile int *flags = S.flags;
-  while (true) {
-    if (threadIdx.x == 0) {
-      task = atomicAdd(S.next_task, 1);
-      ok = (task < S.ntasks && flags[0] == 0) ? 1 : 0;
-      if (ok) ok = wait_task(S, S.tasks[task], flags) ? 1 : 0;
+// Diagonal tiles J = first, first + kDiagBlocks, ...: the tile, updated by
+// the columns before J-1, loses panel (J, J-1) column by column as it is
+// published, then it is factored.  The packed lower triangle sits in
+// registers meanwhile (rows 31-s and s-1 in the lanes of slot s, 17 slots on
+// eight warps); the ninth warp polls.
+constexpr int kSlots = 17;
+__device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, volatile int *flags) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = tid >> 3, q = tid & 7;
+  const TrailEntries te = trail_entries(warp, lane);
+  if (tid == kComputeThreads) sm.fail = 0;
+  for (int J = first; J < S.nt; J += kDiagBlocks) {
+    const bool fed = J > 0 && S.ftile[J] < J;
+    if (warp == 8 && lane == 0) {
+      if (fed && !wait_geq(S.upd + slot_of(S, J, 0), J - 1 - S.ftile[J], flags)) sm.fail = 1;
       __threadfence();
     }
     __syncthreads();
-    if (!ok) break;
-    const int4 t = S.tasks[task];
-    bool fine = true;
-    if (t.x == 0) {
-      fine = factor_diag(S, t.w, sA, flags);
-    } else if (t.x == 1) {
-      panel_solve(S, t.w, t.y - t.w, t.z, sA, sB);
-    } else if (t.x == 2) {
-      pair_update(S, t.w, t.y - t.w, t.z - t.w, sA, sB);
-    } else if (t.x == 4) {
-      fine = chain_task(S, t.w, sC, flags);
-    } else if (t.x == 5) {
-      fine = panel_update_task(S, t.w, t.z, sA, sB, flags);
-    } else if (t.x == 7) {
-      if (S.fwd_nrhs > 0) fine = forward_row(S, t.w, reinterpret_cast<double (*)[kT]>(&sA[0][0]),
-                                             flags);
-    } else {
-      coupling_task(S, t.w, sA, sB, sC, flags);
+    if (sm.fail) return;
+    const double *tile = tile_at(S, J, 0);
+    if (fed) {
+      if (warp == 8) {
+        const double *wl = S.wlstream + (size_t)(J - 1) * 2 * kTT;
+        double a = ld_relaxed(wl + lane), b = ld_relaxed(wl + kT + lane);
+        for (int c = 0; c < kT; c++) {
+          // L is published after P: once it is there, P is a load away
+          if (unset(b)) {
+            b = await_column(wl + c * 2 * kT + kT + lane, flags);
+            if (unset(a)) a = ld_relaxed(wl + c * 2 * kT + lane);
+          }
+          if (unset(a)) a = await_column(wl + c * 2 * kT + lane, flags);
+          sm.W[c][lane] = a;
+          sm.L[c][lane] = b;
+          if (c + 1 < kT) {
+            a = ld_relaxed(wl + (c + 1) * 2 * kT + lane);
+            b = ld_relaxed(wl + (c + 1) * 2 * kT + kT + lane);
+          }
+          __syncwarp();
+          named_sync(10, kFactorThreads);
+        }
+      } else {
+        int rw[3], kk[3];
+        double m[3], acc[3];
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+          const int s = warp + 8 * u;
+          rw[u] = -1;
+          kk[u] = 0;
+          if (s < kSlots) {
+            if (lane < kT - s) { rw[u] = kT - 1 - s; kk[u] = lane; }
+            else if (s < kSlots - 1) { rw[u] = s - 1; kk[u] = lane - (kT - s); }
+          }
+          m[u] = rw[u] >= 0 ? __ldcg(tile + rw[u] * kT + kk[u]) : 0.0;
+          acc[u] = 0.0;
+        }
+        // the products are summed on their own and taken off once, as the
+        // tile pairs' are: one rounding at the size of the tile's entry
+        for (int c = 0; c < kT; c++) {
+          named_sync(10, kFactorThreads);
+#pragma unroll
+          for (int u = 0; u < 3; u++)
+            if (rw[u] >= 0) acc[u] = fma(sm.W[c][rw[u]], sm.L[c][kk[u]], acc[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 3; u++)
+          if (rw[u] >= 0) sm.A[rw[u]][kk[u]] = m[u] - acc[u];
+      }
+    } else if (tid < kComputeThreads) {
+      for (int k = tid; k < kTT; k += kComputeThreads) sm.A[k >> 5][k & 31] = __ldcg(tile + k);
     }
-    if (!fine) break;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp < 8) eliminate_tile(sm, warp, lane, te, S.lstream + (size_t)J * kTT);
+    __syncthreads();
+    if (tid < kT) {
+      const int eq = J * kT + tid;
+      const double d = sm.L[tid][tid];
+      S.invD[eq] = __drcp_rn(d);
+      S.piv[eq] = d;
+      // ProfileSPDLinDirectSolver.cpp:134-138 (first pivot), :189-199; the
+      // first failing pivot of the tile is reported
+      const bool bad = eq < S.n && ((eq == 0) ? !(d > 0.0)
+                                              : (d == 0.0 || fabs(d) <= S.min_diag_tol));
+      const unsigned which = __ballot_sync(0xffffffffu, bad);
+      if (which && tid == 0) {
+        if (atomicCAS((int *)flags, 0, 4) == 0) {
+          flags[1] = J * kT + __ffs(which) - 1;
+          __threadfence();
+          flags[0] = 3;
+        }
+        sm.fail = 1;
+      }
+    }
+    if (tid < kComputeThreads) {
+      double v[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) v[i] = 4 * q + i > r ? 0.0 : sm.L[4 * q + i][r];
+      double2 *g = reinterpret_cast<double2 *>(tile_at(S, J, 0) + r * kT + 4 * q);
+      g[0] = make_double2(v[0], v[1]);
+      g[1] = make_double2(v[2], v[3]);
+    }
+    __syncthreads();
+    if (sm.fail) return;
+    if (tid == 0) {
       __threadfence();
-      if (t.x == 2) atomicAdd(S.upd + slot_of(S, t.y, t.y - t.z), 1);
-      if (t.x == 0 || t.x == 4) atomicExch(S.done + slot_of(S, t.y, 0), 1);
-      if (t.x == 1) atomicAdd(S.done + slot_of(S, t.y, t.y - t.w), 1);
+      atomicExch(S.done + slot_of(S, J, 0), 1);
     }
-    __syncthreads();
   }
 }
 
-// Forward (L y = b), diagonal (z = D^-1 y) and backward (L' x = z)
-// substitution in one block of 1024 threads; x[r * ldx + i] for right-hand
-// side r.  Warp w owns row w of every tile and lane c its column, so a
-// tile's 32 x 32 entries come in with one coalesced load per thread; a step
-// (one tile row forward, one tile column backward) issues the loads of up
-// to kChunk tiles at once, keeps the last W+1 solved tiles of every
-// right-hand side in shared memory, and solves the diagonal tile with warp
-// shuffles.  A step costs about one L2 latency plus the 32-step solve.
-constexpr int kChunk = 24;
-constexpr int kSolveBlock = 1024;
+// Panels (J+1, J) for J = first, first + kPanelBlocks, ...
+__device__ void panel_block(const ProfileSystem &S, FactorSmem &sm, int first,
+                            volatile int *flags) {
+  const int tid = threadIdx.x;
+  for (int J = first; J + 1 < S.nt; J += kPanelBlocks) {
+    if (S.ftile[J + 1] > J) continue;
+    if (tid == 0) {
+      sm.fail = !((J < kRing || wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags)) &&
+                  wait_geq(S.upd + slot_of(S, J + 1, 1), J - max(S.ftile[J + 1], S.ftile[J]),
+                           flags));
+      __threadfence();
+    }
+    __syncthreads();
+    if (sm.fail) return;
+    if (tid < kComputeThreads) panel_task(S, sm, J + 1, J, tid, S.wlstream + (size_t)J * 2 * kTT);
+    else panel_poll(S, sm, J, tid & 31, flags);
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicExch(S.done + slot_of(S, J + 1, 1), 1);
+    }
+  }
+}
 
-__global__ void __launch_bounds__(kSolveBlock) k_prof_solve(ProfileSystem S, int nrhs,
-                                                             double *x, int ldx) {
-  extern __shared__ double win[];                 // [nrhs][W+1][32]
-  __shared__ double red[4][kT][kT + 1];
-  __shared__ double sL[kT][kT + 1];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int nt = S.nt, W = S.W, span = W + 1;
-  auto ywin = [&](int q, int tile) -> double * { return win + ((size_t)q * span + tile % span) * kT; };
-  // ---- forward: t = b_J - sum_o L(J, J-o) y_{J-o}; then unit-lower solve
-  for (int J = 0; J < nt; J++) {
-    const double dval = __ldg(tile_at(S, J, 0) + w * kT + lane);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const int ohi = min(W, J - S.ftile[J]);
-    for (int o0 = 1; o0 <= ohi; o0 += kChunk) {
-      double l[kChunk];
-#pragma unroll
-      for (int k = 0; k < kChunk; k++)
-        l[k] = (o0 + k <= ohi) ? __ldg(tile_at(S, J, o0 + k) + w * kT + lane) : 0.0;
-#pragma unroll
-      for (int k = 0; k < kChunk; k++) {
-        if (o0 + k > ohi) break;
-        for (int q = 0; q < nrhs; q++) acc[q] += l[k] * ywin(q, J - o0 - k)[lane];
+// The other blocks: tasks from the list.  Warp 8 draws the next task and
+// waits for its operands while warps 0-7 run the present one (barriers 7-8:
+// a task is ready, 5-6: its slot is free again); during a panel, which lasts
+// as long as its column's elimination, it polls the column instead.
+__device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, volatile int *flags) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 8) {
+    int pending = 0;
+    bool last_long = false;
+    for (int it = 0;; it++) {
+      const int s = it & 1;
+      while (pending == 2 || (pending && last_long)) {
+        named_sync(5 + ((it - pending) & 1), kFactorThreads);
+        pending--;
       }
-    }
-    for (int q = 0; q < nrhs; q++) {
-      double v = acc[q];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) red[q][0][w] = v;
-    }
-    sL[w][lane] = dval;
-    __syncthreads();
-    if (w < nrhs) {
-      const int q = w;
-      double v = x[(size_t)q * ldx + J * kT + lane] - red[q][0][lane];
-      for (int c = 0; c < kT - 1; c++) {
-        const double yc = __shfl_sync(0xffffffffu, v, c);
-        if (lane > c) v -= sL[lane][c] * yc;
+      int type = -1;
+      if (lane == 0) {
+        const int k = atomicAdd(S.next_task, 1);
+        int4 tk = make_int4(-1, 0, 0, 0);
+        if (k < S.ntasks && flags[0] == 0) {
+          tk = S.tasks[k];
+          if (!wait_task(S, tk, flags)) tk.x = -1;
+        }
+        sm.task[s] = tk;
+        type = tk.x;
+        __threadfence();
       }
-      ywin(q, J)[lane] = v;
-      x[(size_t)q * ldx + J * kT + lane] = v;
+      type = __shfl_sync(0xffffffffu, type, 0);
+      __syncwarp();
+      named_arrive(7 + s, kFactorThreads);
+      if (type < 0) return;
+      if (type == kPanel) panel_poll(S, sm, sm.task[s].w, lane, flags);
+      last_long = type == kPanel;
+      pending++;
     }
-    __syncthreads();
   }
-  // ---- diagonal
-  for (int q = 0; q < nrhs; q++)
-    for (int i = tid; i < nt * kT; i += kSolveBlock) x[(size_t)q * ldx + i] *= S.invD[i];
+  for (int it = 0;; it++) {
+    const int s = it & 1;
+    named_sync(7 + s, kFactorThreads);
+    const int4 t = sm.task[s];
+    if (t.x < 0) return;
+    if (t.x == kPanel) panel_task(S, sm, t.y, t.w, tid, nullptr);
+    else if (t.x == kPair) pair_task(S, t.w, t.y - t.w, t.z - t.w, tid);
+    else if (t.x == kInverse) inverse_task(S, sm, t.w, tid);
+    else if (t.x == kCouple) coupling_task(S, sm, t.w, t.z, tid);
+    else if (t.x == kCouple2) second_coupling_task(S, sm, t.w, t.z, tid);
+    else if (S.fwd_nrhs > 0) forward_row(S, t.w, reinterpret_cast<double (*)[kT]>(&sm.A[0][0]), flags);
+    csync();
+    if (tid == 0) {
+      __threadfence();
+      if (t.x == kPanel) {
+        atomicExch(S.done + slot_of(S, t.y, t.y - t.w), 1);
+      } else if (t.x == kPair) {
+        atomicAdd(S.upd + slot_of(S, t.y, t.y - t.z), 1);
+        atomicAdd(S.colcnt + t.w, 1);
+      } else if (t.x == kInverse) {
+        atomicExch(S.cplw + t.w, 1);
+      } else if (t.x == kCouple) {
+        atomicAdd(S.cpl + t.w, 1);
+      } else if (t.x == kCouple2 && t.z == 0) {
+        atomicExch(S.cplq + t.w, 1);
+      }
+    }
+    __syncwarp();
+    named_arrive(5 + s, kFactorThreads);
+  }
+}
+
+__global__ void __launch_bounds__(kFactorThreads, 1) k_prof_factor(ProfileSystem S) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  FactorSmem &sm = *reinterpret_cast<FactorSmem *>(dyn);
+  __shared__ int ticket;
+  volatile int *flags = S.flags;
+  if (threadIdx.x == 0) ticket = atomicAdd(S.next_task + 1, 1);
   __syncthreads();
-  // ---- backward: t = z_J - sum_o L(J+o, J)' x_{J+o}; then unit-upper solve
-  for (int J = nt - 1; J >= 0; J--) {
-    const double dval = __ldg(tile_at(S, J, 0) + w * kT + lane);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const int ohi = min(W, nt - 1 - J);
-    for (int o0 = 1; o0 <= ohi; o0 += kChunk) {
-      double l[kChunk];
-#pragma unroll
-      for (int k = 0; k < kChunk; k++)
-        l[k] = (o0 + k <= ohi && S.ftile[J + o0 + k] <= J)
-                   ? __ldg(tile_at(S, J + o0 + k, o0 + k) + w * kT + lane)
-                   : 0.0;
-      // row w of tile (J+o, J) times x_{J+o}[w]; summed over rows below
-#pragma unroll
-      for (int k = 0; k < kChunk; k++) {
-        if (o0 + k > ohi) break;
-        for (int q = 0; q < nrhs; q++) acc[q] += l[k] * ywin(q, J + o0 + k)[w];
-      }
-    }
-    for (int q = 0; q < nrhs; q++) red[q][w][lane] = acc[q];
-    sL[w][lane] = dval;
-    __syncthreads();
-    if (w < nrhs) {
-      const int q = w;
-      double sum = 0.0;
-      for (int h = 0; h < kT; h++) sum += red[q][h][lane];
-      double v = x[(size_t)q * ldx + J * kT + lane] - sum;
-      // x_c = v_c - sum_{k > c} L[k][c] x_k, from the last row up
-      for (int cc = kT - 1; cc > 0; cc--) {
-        const double xc = __shfl_sync(0xffffffffu, v, cc);
-        if (lane < cc) v -= sL[cc][lane] * xc;
-      }
-      ywin(q, J)[lane] = v;
-      x[(size_t)q * ldx + J * kT + lane] = v;
-    }
-    __syncthreads();
-  }
+  if (ticket < kDiagBlocks) diag_block(S, sm, ticket, flags);
+  else if (ticket < kDiagBlocks + kPanelBlocks) panel_block(S, sm, ticket - kDiagBlocks, flags);
+  else worker_block(S, sm, flags);
 }
 
 __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem S, int nrhs,
-                                                                  double *x, int ldx,
                                                                   double *ys, double *cs,
                                                                   double *xs, double *ds,
                                                                   int backward_only) {
   __shared__ double rv[2][4][kT];
   volatile int *flags = S.flags;
+  if (flags[0] != 0) return;                    // the factorisation failed
   const int tid = threadIdx.x;
   const int r = tid >> 3, g = tid & 7;          // tile row, column group (4 columns)
   const int nt = S.nt, W = S.W, P = gridDim.x, ls = nt * kT;
@@ -830,7 +1054,7 @@ __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem 
     double(*rb)[kT] = rv[it & 1];
     for (int q = 0; q < nrhs; q++) {
       const double v = group_sum(acc[q]);
-      if (g == 0) rb[q][r] = __ldcg(x + (size_t)q * ldx + J * kT + r) - v;
+      if (g == 0) rb[q][r] = rhs_at(S, q, J * kT + r) - v;
     }
     const double *Wt = S.Winv + (size_t)J * kTT;
     double wv[4];
@@ -910,7 +1134,7 @@ __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem 
       if (g == 0) {
         const double xj = (c3 - t1) - t2;
         publish(xs + vq + J * kT + r, xj);
-        x[(size_t)q * ldx + J * kT + r] = xj;
+        if (J * kT + r < S.n) S.x[q][J * kT + r] = xj;
       }
     }
   }
@@ -937,150 +1161,121 @@ int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &
   return 0;
 }
 
-// The dataflow order of the factor tasks (type, I, K, J): type 0 diagonal
-// tile J (I = K = J), 1 rows 8K..8K+7 of panel tile (I, J), 2 update of
-// tile (I, K) by
-// column J, 3 the update of diagonal tile J+1 by column J followed by its
-// factorisation (it is that tile's last update).
-void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks) {
+// The dataflow order of the list's tasks (type, I, K, J): the stream's blocks
+// run the diagonal tiles and the panels (J+1, J).  Column J: the updates of
+// column J-1 that reach column J+1 (the next diagonal tile's last but one
+// first), panel (J+2, J) and its update of tile (J+2, J+1) -- what the stream
+// waits for next --, the other panels, column J's updates of column J+1, the
+// rest of column J-1's trailing update, and the coupling matrices and
+// forward step two columns back.  npairs: tile pairs of each column.
+void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks,
+                   std::vector<int> &npairs) {
   tasks.clear();
+  npairs.assign(std::max(nt, 1), 0);
   auto emit = [&](int type, int I, int K, int J) {
     tasks.push_back(type); tasks.push_back(I); tasks.push_back(K); tasks.push_back(J);
+    if (type == kPair) npairs[J]++;
   };
-  // the updates of column J (0 <= J < nt) whose target column is J+b for b
-  // in [blo, bhi]
-  // (the pair (J+1, J+1) of column J belongs to column J's chain task)
-  auto updates = [&](int J, int blo, int bhi) {
+  // the updates of column J whose target column is J+b for b in [blo, bhi]
+  // from row J+alo on (the pair (J+1, J+1) belongs to the stream)
+  auto updates = [&](int J, int blo, int bhi, int alo) {
     if (J < 0) return;
     const int omax = std::min(W, nt - 1 - J);
     for (int b = blo; b <= std::min(bhi, omax); b++) {
       if (ftile[J + b] > J) continue;
-      for (int a = b; a <= omax; a++)
-        if (ftile[J + a] <= J && !(a == 1 && b == 1)) emit(2, J + a, J + b, J);
+      for (int a = std::max(b, alo); a <= omax; a++)
+        if (ftile[J + a] <= J) emit(kPair, J + a, J + b, J);
     }
   };
-  // Column J: the updates of column J-1 that reach column J+1 (the
-  // diagonal's included), the chain task (panel (J+1, J), the last update
-  // and the LDL' of diagonal tile J+1), the other panels, column J's
-  // updates of column J+1, then the rest of column J-1's trailing update.
+  auto couple = [&](int J) {
+    if (J < 0) return;
+    emit(kInverse, J, J, J);
+    for (int p = 0; p < 4; p++) emit(kCouple, J, p, J);
+    emit(kCouple2, J, 0, J);
+    if (J >= 1) emit(kCouple2, J - 1, 1, J - 1);
+    if (J == nt - 1) emit(kCouple2, J, 1, J);
+    emit(kForward, J, J, J);
+  };
   for (int J = 0; J < nt; J++) {
-    if (ftile[J] == J) emit(0, J, J, J);   // no column updates this tile
-    updates(J - 1, 2, 2);
+    updates(J - 1, 2, 2, 2);
     const int omax = std::min(W, nt - 1 - J);
-    if (omax >= 1 && ftile[J + 1] <= J)
-      for (int q = 0; q < kPanelParts; q++) emit(5, J + 1, q, J);
-    if (J + 1 < nt && ftile[J + 1] <= J) emit(4, J + 1, J + 1, J);
-    for (int o = 2; o <= omax; o++)
-      if (ftile[J + o] <= J)
-        for (int q = 0; q < kPanelParts; q++) emit(1, J + o, q, J);
-    updates(J, 1, 1);
-    updates(J - 1, 3, W);
-    if (J >= 2) {
-      emit(6, J - 2, J - 2, J - 2);
-      emit(7, J - 2, J - 2, J - 2);
+    if (omax >= 2 && ftile[J + 2] <= J) {
+      emit(kPanel, J + 2, J + 2, J);
+      if (ftile[J + 1] <= J) emit(kPair, J + 2, J + 1, J);
     }
+    for (int o = 3; o <= omax; o++)
+      if (ftile[J + o] <= J) emit(kPanel, J + o, J + o, J);
+    updates(J, 1, 1, 3);
+    updates(J - 1, 3, W, 3);
+    couple(J - 2);
   }
-  updates(nt - 1, 2, W);
-  for (int J = std::max(nt - 2, 0); J < nt; J++) {
-    emit(6, J, J, J);
-    emit(7, J, J, J);
-  }
+  for (int J = std::max(nt - 2, 0); J < nt; J++) couple(J);
 }
 
 size_t profile_tile_doubles(int nt, int W) { return (size_t)nt * (W + 1) * kTT; }
+size_t profile_digit_bytes(int W) { return (size_t)kRing * W * kSlotBytes; }
 int profile_tile_edge() { return kT; }
 
-int profile_factor(const ProfileSystem &S, cudaStream_t s, int *bad_eq) {
+int profile_factor(const ProfileSystem &S, cudaStream_t s) {
   if (S.n == 0) return 0;
-  if (cudaMemsetAsync(S.L, 0, profile_tile_doubles(S.nt, S.W) * sizeof(double), s) != cudaSuccess)
-    return XG_ECUDA;
-  const int fill_threads = 256;
-  const long warps = (long)S.nt * kT;
-  k_prof_fill<<<(int)((warps * 32 + fill_threads - 1) / fill_threads), fill_threads, 0, s>>>(S);
-  if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
   if (g_factor_blocks < 0) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_prof_factor, kFactorThreads, 0);
-    if (per < 1) per = 1;
-    // one block per SM: a block that runs a task on the critical path (a
-    // diagonal tile, a panel) must not share its SM's few FP64 units with a
-    // bulk tile update; the dynamic shared memory requested below keeps a
-    // second block off the SM
-    g_factor_blocks = sms;
-    cudaFuncSetAttribute(k_prof_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kFactorSoloSmem);
-  }
-  const size_t nslots = (size_t)S.nt * (S.W + 1);
-  if (S.fwd_nrhs > 0) {
-    // the forward sweep runs inside: its published values start unset
-    if (!profile_pipelined(S) || S.fwd_nrhs > 4 || !S.fwd_x) return XG_EINVAL;
-    const size_t ls = (size_t)S.nt * kT;
-    if (cudaMemsetAsync(S.sweep, 0xFF, 2 * (size_t)S.fwd_nrhs * ls * sizeof(double), s) !=
-        cudaSuccess)
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(k_prof_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kFactorSmem) != cudaSuccess)
       return XG_ECUDA;
+    g_factor_blocks = sms;
   }
-  if (cudaMemsetAsync(S.upd, 0, nslots * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  if (cudaMemsetAsync(S.done, 0, nslots * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  if (cudaMemsetAsync(S.cpl, 0, (size_t)S.nt * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  if (cudaMemsetAsync(S.next_task, 0, sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  if (cudaMemsetAsync(S.flags, 0, 4 * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  const int nb = (int)std::min<long>(g_factor_blocks, std::max(S.ntasks, 1));
-  k_prof_factor<<<nb, kFactorThreads, kFactorSoloSmem, s>>>(S);
+  if (S.fwd_nrhs < 0 || S.fwd_nrhs > 4) return XG_EINVAL;
+  // the sweeps' values: forward ones published inside the factorisation,
+  // backward ones by the solve behind it
+  const size_t nsweep = 4 * (size_t)S.fwd_nrhs * S.nt * kT;
+  const long nprep = std::min<long>(8 * (long)g_factor_blocks, (long)S.nt * kT / 8);
+  k_prof_prepare<<<(int)std::max<long>(nprep, 1), 256, 0, s>>>(S, S.counter_bytes / sizeof(int),
+                                                               nsweep);
   if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
+  // all blocks co-resident: the stream waits for list tasks and they for it
+  const int nb = (int)std::min<long>(g_factor_blocks, kDiagBlocks + kPanelBlocks + (long)S.ntasks);
+  if (nb <= kDiagBlocks + kPanelBlocks) return XG_ECUDA;
+  ProfileSystem Sv = S;
+  void *args[] = {(void *)&Sv};
+  return cudaLaunchCooperativeKernel((void *)k_prof_factor, dim3(nb), dim3(kFactorThreads), args,
+                                     kFactorSmem, s) == cudaSuccess
+             ? 0 : XG_ECUDA;
+}
+
+int profile_status(const ProfileSystem &S, cudaStream_t s, int *bad_eq) {
+  if (bad_eq) *bad_eq = -1;
+  if (S.n == 0) return 0;
   int hflags[4];
   if (cudaMemcpyAsync(hflags, S.flags, sizeof hflags, cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return XG_ECUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return XG_ECUDA;
-  if (bad_eq) *bad_eq = hflags[0] == 3 ? hflags[1] : -1;
-  if (hflags[0] == 3) return XG_ESOLVE;   // pivot check failed
-  if (hflags[0] != 0) return XG_ESOLVE;   // a dependency wait timed out
-  return 0;
+  if (bad_eq && hflags[0] == 3) *bad_eq = hflags[1];
+  return hflags[0] != 0 ? XG_ESOLVE : 0;   // a pivot check failed, or a wait timed out
 }
 
-bool profile_pipelined(const ProfileSystem &S) { return S.sweep && S.nt >= 2 * kPipeBlocks; }
-
-int profile_solve(const ProfileSystem &S, int nrhs, double *x, int ldx, cudaStream_t s,
-                  bool backward_only) {
+int profile_solve(const ProfileSystem &S, int nrhs, cudaStream_t s, bool backward_only) {
   if (S.n == 0) return 0;
-  if (nrhs < 1 || nrhs > 4 || ldx < S.nt * kT) return XG_EINVAL;
-  if (backward_only && !profile_pipelined(S)) return XG_EINVAL;
-  if (profile_pipelined(S)) {
-    // pipelined over co-resident blocks (the sweeps' published values are
-    // reset to kUnset first; after a factorisation that ran the forward
-    // sweep, only the backward sweep's); small systems keep the one-block
-    // sweep
-    const size_t ls = (size_t)S.nt * kT;
-    double *ys = S.sweep, *cs = ys + (size_t)nrhs * ls, *xs = cs + (size_t)nrhs * ls;
-    double *ds = xs + (size_t)nrhs * ls;
-    double *reset = backward_only ? xs : ys;
-    const size_t nreset = (backward_only ? 2 : 4) * (size_t)nrhs * ls;
-    if (cudaMemsetAsync(reset, 0xFF, nreset * sizeof(double), s) != cudaSuccess)
+  if (nrhs < 1 || nrhs > 4) return XG_EINVAL;
+  const size_t ls = (size_t)S.nt * kT;
+  double *ys = S.sweep, *cs = ys + (size_t)nrhs * ls, *xs = cs + (size_t)nrhs * ls;
+  double *ds = xs + (size_t)nrhs * ls;
+  // the sweeps' published values start unset (behind a factorisation that ran
+  // the forward sweep they are)
+  if (!backward_only) {
+    if (cudaMemsetAsync(ys, 0xFF, 4 * (size_t)nrhs * ls * sizeof(double), s) != cudaSuccess)
       return XG_ECUDA;
     if (cudaMemsetAsync(S.flags, 0, 4 * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-    ProfileSystem Sv = S;
-    int bonly = backward_only ? 1 : 0;
-    void *args[] = {(void *)&Sv, (void *)&nrhs, (void *)&x,  (void *)&ldx, (void *)&ys,
-                    (void *)&cs, (void *)&xs,   (void *)&ds, (void *)&bonly};
-    if (cudaLaunchCooperativeKernel((void *)k_prof_solve_pipe, dim3(kPipeBlocks),
-                                    dim3(kPipeThreads), args, 0, s) != cudaSuccess)
-      return XG_ECUDA;
-    int hflag = 0;
-    if (cudaMemcpyAsync(&hflag, S.flags, sizeof hflag, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-      return XG_ECUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return XG_ECUDA;
-    return hflag != 0 ? XG_ESOLVE : 0;   // a sweep wait timed out
   }
-  const size_t win = (size_t)nrhs * (S.W + 1) * kT * sizeof(double);
-  const size_t stat = (4 * kT * (kT + 1) + kT * (kT + 1)) * sizeof(double);
-  if (win + stat > 227 * 1024)
-    return XG_EINVAL;   // envelope wider than the substitution window
-  if (cudaFuncSetAttribute(k_prof_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)win) != cudaSuccess)
-    return XG_ECUDA;
-  k_prof_solve<<<1, kSolveBlock, win, s>>>(S, nrhs, x, ldx);
-  return cudaGetLastError() == cudaSuccess ? 0 : XG_ECUDA;
+  ProfileSystem Sv = S;
+  int bonly = backward_only ? 1 : 0;
+  void *args[] = {(void *)&Sv, (void *)&nrhs, (void *)&ys, (void *)&cs,
+                  (void *)&xs, (void *)&ds,   (void *)&bonly};
+  return cudaLaunchCooperativeKernel((void *)k_prof_solve_pipe, dim3(std::min(kPipeBlocks, S.nt)),
+                                     dim3(kPipeThreads), args, 0, s) == cudaSuccess
+             ? 0 : XG_ECUDA;
 }
 
 }  // namespace xg
