@@ -9,18 +9,14 @@
 // Storage: part c, local row i holds the entries (i, i-k), k = 0..b_c, at
 // band[boff[c] + i*(b_c+1) + k] (b_c: the part's envelope width).
 //
-// Factor (k_band_factor_win): right-looking.  The rows column j touches,
-// j..j+b, live in a ring of shared-memory rows; the rows beyond them are
-// fetched kBandAhead columns early with cp.async, and a finished row goes
-// back to the band.  Column j takes two barriers: the threads below the
-// pivot scale the column (l = a / d) and apply it to the right-hand sides,
-// then the trailing triangle takes one FMA per entry, and the threads that
-// finish column j+1's entries hand them (and the next pivot's reciprocal) to
-// the next column through a second buffer.  The forward substitution and
-// the diagonal scaling of up to four right-hand sides run inside the
-// factorisation; the backward substitution (k_band_back) is one warp per
-// part walking the band's rows upwards (x_i final, then the rows above take
-// one FMA each from row i of L), rows prefetched the same way.
+// Factor (k_band_factor): right-looking, the pivot chain one column ahead of
+// the trailing update.  The rows column j touches, j..j+b, live in a ring of
+// shared-memory rows; the rows beyond them are fetched kBandAhead columns
+// early with cp.async, and a finished row goes back to the band.  The forward
+// substitution and the diagonal scaling of up to four right-hand sides run
+// inside the factorisation; the backward substitution (k_band_back) is one
+// warp per part walking the band's rows upwards (x_i final, then the rows
+// above take one FMA each from row i of L), rows prefetched the same way.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,12 +28,12 @@ namespace xg {
 
 namespace {
 
-constexpr int kBandWorkers = 96;        // warps 1-3
-constexpr int kBandThreads = kBandWorkers + 32;
-constexpr int kBandMaxWidth = 255;      // widest envelope band_plan accepts
+constexpr int kBandTrail = 6;           // trailing warps
+constexpr int kBandWorkers = 32 * kBandTrail;
+constexpr int kBandThreads = kBandWorkers + 64;
+constexpr int kBandMaxWidth = 77;       // widest envelope band_plan accepts
 constexpr int kBandAhead = 8;           // rows fetched ahead of use
 constexpr int kBandMaxRhs = 4;
-constexpr int kBackWarps = 4;
 
 // reciprocal on the pivot chain (xg_rcp.h); the stored reciprocals are the
 // correctly rounded ones
@@ -74,162 +70,213 @@ __device__ __forceinline__ bool pivot_fails(const BandSystem &S, int j, double d
   return (j == 0) ? !(d > 0.0) : (d == 0.0 || fabs(d) <= S.min_diag_tol);
 }
 
-// Shared memory (doubles): W[R*ldm] ring rows, Y[R*kBandMaxRhs] ring of the
-// right-hand sides, col[2*ldm], lcol[ldm].  ldm = bmax + 1, R = the power of
-// two at or above ldm + kBandAhead (ring slot = row & (R-1)).
-// Warps 1-3 scale the columns and update the trailing triangles; warp 0
-// carries the pivot chain (the next pivot's last update right after the
-// column is scaled, its reciprocal while the others update), the
-// right-hand sides (forward substitution) and their ring.  Every worker
-// owns up to K entries (ti, tk) of the width-b trailing triangle, fixed for
-// the whole factorisation (entry q = worker + 96 k, row-major); a column
-// loads all its entries' operands before their FMAs.
-template <int K>
-__global__ void __launch_bounds__(kBandThreads) k_band_factor_win(BandSystem S, int nrhs,
-                                                                   double *x, int ldx, int R) {
+__device__ __forceinline__ void band_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void band_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// A window of 32 NB consecutive rows over a warp: row r sits in lane r % 32,
+// register (r / 32) % NB.
+template <int NB>
+__device__ __forceinline__ double window_row(const double (&v)[NB], int r) {
+  double t = v[0];
+  if (NB == 2) t = (r & 32) ? v[NB - 1] : v[0];
+  if (NB == 4) {
+    const double a = (r & 32) ? v[1 % NB] : v[0], b = (r & 32) ? v[NB - 1] : v[2 % NB];
+    t = (r & 64) ? b : a;
+  }
+  return __shfl_sync(0xffffffffu, t, r & 31);
+}
+
+// Shared memory (doubles): W[R*ldm] ring rows (entry (r, r-k) at (r % R)*ldm +
+// k; ldm = bmax + 1, R a power of two: ring_rows), lcol and ccol [4][32 NB] the
+// last columns of L and of the unscaled columns, by row, Yr
+// [2*kBandAhead][kBandMaxRhs] right-hand sides on their way in.
+//
+// Warp 0 carries the pivot chain: with column j final it takes the pivot's
+// reciprocal, scales the column, applies it to column j+1 (rows in registers,
+// NB of them a lane; the raw column from the ring) and hands both on.  Warps
+// 1-6 apply column j to columns j+2 and beyond, one FMA per entry, each thread
+// up to K fixed entries (ti, tk) of the width-b trailing triangle in
+// column-major order, so that column j+2, which the chain waits for, is every
+// thread's first.  Warp 7 carries the right-hand sides (forward substitution,
+// rows in registers as well), writes finished rows back and fetches new ones.
+// Named barriers 1-2 (chain -> all, by column parity) and 3-4 (trailing ->
+// chain).  One warp gets an FP64 operation every 64 cycles and the SM one every
+// 19: a column of a 42-wide band (28 trailing operations, 7 on the chain) is
+// bound by the unit at about 700 cycles, a narrow one by the chain at 550; with
+// two block barriers a column and three trailing warps it took 1,860.  Every
+// entry takes the same FMAs in the same order as before, bit for bit.
+template <int K, int NB>
+__global__ void __launch_bounds__(kBandThreads) k_band_factor(BandSystem S, int nrhs, double *x,
+                                                              int ldx, int R) {
   extern __shared__ double sm[];
   const int c = blockIdx.x;
   if (c >= S.ncomp) return;
   const int e0 = S.cstart[c], n = S.cstart[c + 1] - e0, b = S.bw[c], ld = b + 1;
   const int ldm = S.bmax + 1, Rm = R - 1;
+  constexpr int kWin = 32 * NB, kMask = kWin - 1;
   double *W = sm;
-  double *Y = W + (size_t)R * ldm;
-  double *colb = Y + (size_t)R * kBandMaxRhs;
-  double *lcol = colb + 2 * ldm;
-  __shared__ double sinv[2], pivv;
+  double *lcol = W + (size_t)R * ldm, *ccol = lcol + 4 * kWin;
+  double *Yr = ccol + 4 * kWin;
   __shared__ int bad;
-  const int tid = threadIdx.x;
-  const bool worker = tid >= 32;
-  const int wid = tid - 32;                     // worker index
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double *B = S.band + S.boff[c];
   band_fill(S, e0, n, ld, B);
-  // this worker's entries: q = wid + 96 k of the row-major lower triangle
-  // of width b, without entry 0 (the pivot, warp 0's), as (ti << 16) | tk
-  int ent[K];
-  const int trib = b * (b + 1) / 2;
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const int q = wid + kBandWorkers * k;
-    ent[k] = -1;
-    if (worker && q > 0 && q < trib) {
-      int ti = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
-      while (ti * (ti + 1) / 2 > q) ti--;
-      while ((ti + 1) * (ti + 2) / 2 <= q) ti++;
-      ent[k] = (ti << 16) | (q - ti * (ti + 1) / 2);
-    }
-  }
-  // the first R rows and their right-hand sides directly
   const int n0 = min(n, R);
   for (int k = tid; k < n0 * ld; k += blockDim.x) W[(k / ld) * ldm + k % ld] = B[k];
-  for (int k = tid; k < n0 * nrhs; k += blockDim.x)
-    Y[(k / nrhs) * kBandMaxRhs + k % nrhs] = x[(long)(k % nrhs) * ldx + e0 + k / nrhs];
   if (tid == 0) bad = 0;
   __syncthreads();
-  // column 0's entries and pivot
-  for (int t = tid; t < min(b, n - 1); t += blockDim.x) colb[t] = W[(1 + t) * ldm + 1 + t];
-  if (tid == 0 && n > 0) {
-    const double d = W[0];
-    if (pivot_fails(S, 0, d)) {
+  constexpr int kAll = kBandThreads, kBack = kBandWorkers + 32;
+  if (warp == 0) {
+    double xc[NB];                // column j by rows, zero outside the band
+    double d = n > 0 ? W[0] : 1.0;
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const int r = 1 + ((lane + 32 * u - 1) & kMask);
+      xc[u] = r <= min(b, n - 1) ? W[(r & Rm) * ldm + r] : 0.0;
+    }
+    if (lane == 0 && n > 0 && pivot_fails(S, 0, d)) {
       bad = 1;
       S.flags[1] = e0;
       S.flags[0] = 3;
     }
-    sinv[0] = chain_rcp(d);
-  }
-  __syncthreads();
-  for (int j = 0; j < n; j++) {
-    const int m = min(b, n - 1 - j);
-    const int sj = j & Rm, s1 = (j + 1) & Rm;
-    const double *cl = colb + (j & 1) * ldm;
-    double *cn = colb + ((j + 1) & 1) * ldm;
-    double *Wj = W + sj * ldm;
-    const double inv = sinv[j & 1];
-    if (worker) {
-      // scale the column
-      for (int t = wid; t < m; t += kBandWorkers) {
-        const double l = cl[t] * inv;
-        lcol[t] = l;
-        W[((s1 + t) & Rm) * ldm + 1 + t] = l;
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      const double inv = chain_rcp(d);
+      if (j >= 1) band_sync(3 + ((j - 1) & 1), kBack);
+      // raw column j+1, rows j+1 .. min(j+1+b, n-1)
+      int r[NB];
+      double raw[NB];
+      const int last = min(j + 1 + b, n - 1);
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        r[u] = j + 1 + ((lane + 32 * u - (j + 1)) & kMask);
+        raw[u] = r[u] <= last ? W[(r[u] & Rm) * ldm + r[u] - (j + 1)] : 0.0;
       }
-    } else if (tid == 0 && m > 0) {
-      // the next pivot's last update (the arithmetic of the trailing
-      // triangle's entry (0, 0), which the workers leave out)
-      const double l0 = cl[0] * inv;
-      double *a = W + s1 * ldm;
-      pivv = fma(-l0, cl[0], *a);
-      *a = pivv;
+      const double ucc = window_row<NB>(xc, j + 1);
+      double l[NB], xn[NB];
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        l[u] = xc[u] * inv;
+        xn[u] = r[u] <= j + b ? fma(-l[u], ucc, raw[u]) : raw[u];
+      }
+      double *lc = lcol + (j & 3) * kWin, *cc = ccol + (j & 3) * kWin;
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        lc[r[u] & kMask] = l[u];
+        cc[r[u] & kMask] = xc[u];
+        if (r[u] <= min(j + b, n - 1)) W[(r[u] & Rm) * ldm + r[u] - j] = l[u];
+        if (r[u] == j + 1 && j + 1 < n) W[((j + 1) & Rm) * ldm] = xn[u];
+      }
+      band_arrive(1 + (j & 1), kAll);
+      d = window_row<NB>(xn, j + 1);
+      if (lane == 0 && j + 1 < n && pivot_fails(S, j + 1, d) && !bad) {
+        bad = 1;
+        S.flags[1] = e0 + j + 1;
+        S.flags[0] = 3;
+      }
+#pragma unroll
+      for (int u = 0; u < NB; u++) xc[u] = r[u] == j + 1 ? 0.0 : xn[u];
     }
-    // row j+b+1, fetched kBandAhead columns ago, is complete for everyone
-    // after this barrier
-    cp_async_wait<kBandAhead - 1>();
-    __syncthreads();
-    if (worker) {
-      // trailing triangle (rows and columns j+1..j+m), one FMA per entry
-      double *ap[K];
-      double lv[K], cv[K], av[K];
+  } else if (warp <= kBandTrail) {
+    // entries (ti, tk), 1 <= tk <= ti < b, of the window's triangle,
+    // column-major: (ti << 16) | tk
+    int ent[K];
+    const int wid = tid - 32;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      int q = wid + kBandWorkers * k;
+      ent[k] = -1;
+      for (int tk = 1; tk < b; tk++) {
+        if (q < b - tk) {
+          ent[k] = ((tk + q) << 16) | tk;
+          break;
+        }
+        q -= b - tk;
+      }
+    }
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      band_sync(1 + (j & 1), kAll);
+      const int m = min(b, n - 1 - j);
+      const double *lc = lcol + (j & 3) * kWin, *cc = ccol + (j & 3) * kWin;
+      // one pass of the loop is three loads, an FMA and a store; column j+2 is
+      // in the first pass and released right behind it
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int e = ent[k];
         const int ti = e >> 16, tk = e & 0xffff;
         if (e >= 0 && ti < m) {
-          ap[k] = W + ((s1 + ti) & Rm) * ldm + (ti - tk);
-          lv[k] = lcol[ti];
-          cv[k] = cl[tk];
-          av[k] = *ap[k];
+          const int row = j + 1 + ti;
+          double *a = W + (row & Rm) * ldm + (ti - tk);
+          *a = fma(-lc[row & kMask], cc[(j + 1 + tk) & kMask], *a);
         }
+        if (k == 0 && j < n - 1) band_arrive(3 + (j & 1), kBack);
+      }
+    }
+  } else {
+    // right-hand sides: row r's value in register (r / 32) % NB of lane r % 32
+    double y[NB][kBandMaxRhs];
+#pragma unroll
+    for (int u = 0; u < NB; u++)
+#pragma unroll
+      for (int q = 0; q < kBandMaxRhs; q++) {
+        const int r = lane + 32 * u;
+        y[u][q] = q < nrhs && r < n ? x[(long)q * ldx + e0 + r] : 0.0;
+      }
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      band_sync(1 + (j & 1), kAll);
+      const double *lc = lcol + (j & 3) * kWin;
+      const int m = min(b, n - 1 - j);
+      double lv[NB];
+      bool in[NB];
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const int r = j + 1 + ((lane + 32 * u - (j + 1)) & kMask);
+        in[u] = r <= j + m;
+        lv[u] = in[u] ? lc[r & kMask] : 0.0;
       }
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        const int e = ent[k];
-        const int ti = e >> 16, tk = e & 0xffff;
-        if (e >= 0 && ti < m) {
-          const double v = fma(-lv[k], cv[k], av[k]);
-          *ap[k] = v;
-          if (tk == 0) cn[ti - 1] = v;
+      for (int q = 0; q < kBandMaxRhs; q++) {
+        if (q >= nrhs) break;
+        double col[NB];
+#pragma unroll
+        for (int u = 0; u < NB; u++) col[u] = y[u][q];
+        const double yj = window_row<NB>(col, j);
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+          if (in[u]) y[u][q] = fma(-lv[u], yj, y[u][q]);
+          // row j's slot takes row j + 32 NB, fetched through shared memory:
+          // it arrives kBandAhead columns later, before its first use
+          const double *yi = Yr + ((j - kBandAhead) & (2 * kBandAhead - 1)) * kBandMaxRhs + q;
+          if (lane + 32 * u == ((j - kBandAhead) & kMask) && j >= kBandAhead)
+            y[u][q] = *yi;
+          if (lane + 32 * u == (j & kMask)) {
+            x[(long)q * ldx + e0 + j] = y[u][q];
+            if (j + kWin < n)
+              cp_async8(Yr + (j & (2 * kBandAhead - 1)) * kBandMaxRhs + q,
+                        x + (long)q * ldx + e0 + j + kWin);
+          }
         }
       }
-      // row j is final: back to the band; its ring row then takes band row
-      // j+R (each entry is read and refilled by the same thread)
+      // row j is final: back to the band; its ring row takes band row j+R,
+      // which is complete kBandAhead columns later
       const bool refill = j + R < n;
-      for (int t = wid; t < ld; t += kBandWorkers) {
+      double *Wj = W + (j & Rm) * ldm;
+      for (int t = lane; t < ld; t += 32) {
         B[(long)j * ld + t] = Wj[t];
         if (refill) cp_async8(Wj + t, B + (long)(j + R) * ld + t);
       }
-    } else {
-      if (tid == 0 && m > 0) {
-        const double v = pivv;
-        if (pivot_fails(S, j + 1, v) && atomicCAS(&bad, 0, 1) == 0) {
-          S.flags[1] = e0 + j + 1;
-          S.flags[0] = 3;
-        }
-        sinv[(j + 1) & 1] = chain_rcp(v);
-      }
-      // forward substitution: the right-hand sides below row j take the
-      // column (its entries in lcol, complete after the barrier above)
-      const double *yj = Y + sj * kBandMaxRhs;
-      for (int t = tid; t < m; t += 32) {
-        double *yr = Y + ((s1 + t) & Rm) * kBandMaxRhs;
-        const double l = lcol[t];
-        for (int r = 0; r < nrhs; r++) yr[r] = fma(-l, yj[r], yr[r]);
-      }
+      cp_async_commit();
+      cp_async_wait<kBandAhead - 1>();
       __syncwarp();
-      if (tid == 0) {
-        // row j's forward-substituted right-hand sides (scaled by the
-        // reciprocal pivots after the loop); the ring row takes row j+R
-        double *yw = Y + sj * kBandMaxRhs;
-        for (int r = 0; r < nrhs; r++) {
-          x[(long)r * ldx + e0 + j] = yw[r];
-          if (j + R < n) cp_async8(yw + r, x + (long)r * ldx + e0 + j + R);
-        }
-      }
-      if (b > 0 && j + b + 1 < n && tid == 1)   // column j+1's entry in row j+b+1
-        cn[b - 1] = W[((s1 + b) & Rm) * ldm + b];
     }
-    cp_async_commit();
-    __syncthreads();
-    if (bad) break;
+    cp_async_wait<0>();
   }
-  cp_async_wait<0>();
   __syncthreads();
   // the correctly rounded reciprocal pivots, and the diagonal scaling
   if (!bad) {
@@ -241,62 +288,100 @@ __global__ void __launch_bounds__(kBandThreads) k_band_factor_win(BandSystem S, 
   }
 }
 
-// Backward substitution, one warp per part: x_i = z_i once every row below
-// has been applied, then z_{i-1-t} -= L(i, i-1-t) x_i for t < b (row i of
-// the band, contiguous).  The band rows come through a ring of kBandAhead
-// rows fetched ahead (one row per sweep step, over all right-hand sides in
-// turn); z sits in shared memory when the part has at most zcap equations.
-__global__ void __launch_bounds__(32 * kBackWarps) k_band_back(BandSystem S, int nrhs, double *x,
-                                                               int ldx, int zcap) {
+// Backward substitution of one part per block: x_i = z_i once every row below
+// has been applied, then z_r -= L(i, r) x_i for r = i-1 .. i-b (row i of the
+// band, contiguous), over all right-hand sides in turn.  Warp 0 computes: the
+// rows in reach sit in its registers (window_row), a step is a shuffle and an
+// FMA a register, no branch, its operands in shared memory.  Warp 1 feeds it
+// in batches of kBackRows steps, kBackStages of them in flight (cp.async): the
+// band's rows, and the rows of z that come into reach; it takes the results
+// back.  Named barriers 1-4: a batch is there, 5-8: its place is free.  z
+// through shared memory with the fetching in the same warp took 550 cycles a
+// row; the FMA's way to the shuffle and back is 120.
+constexpr int kBackRows = 8, kBackStages = 4;
+
+size_t back_smem(int bmax) {
+  return (size_t)kBackStages * kBackRows * (bmax + 1 + 2) * sizeof(double);
+}
+
+template <int NB>
+__global__ void __launch_bounds__(64) k_band_back(BandSystem S, int nrhs, double *x, int ldx) {
   extern __shared__ double sm[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * kBackWarps + w;
-  const int ldm = S.bmax + 1;
-  double *rows = sm + (size_t)w * (kBandAhead * ldm + zcap);
-  double *zs = rows + kBandAhead * ldm;
-  if (c >= S.ncomp) return;
+  constexpr int kWin = 32 * NB, kMask = kWin - 1;
+  const int lane = threadIdx.x & 31, c = blockIdx.x, ldm = S.bmax + 1;
+  double *rows = sm;                                              // [stage][step][ldm]
+  double *zin = rows + (size_t)kBackStages * kBackRows * ldm;     // [stage][step]
+  double *xout = zin + kBackStages * kBackRows;                   // [stage][step]
   const int e0 = S.cstart[c], n = S.cstart[c + 1] - e0, b = S.bw[c], ld = b + 1;
   const double *B = S.band + S.boff[c];
-  const long T = (long)nrhs * n;           // sweep steps: rhs k / n, row n-1 - k % n
-  for (long k = 0; k < kBandAhead; k++) {
-    if (k < T) {
-      const long i = n - 1 - k % n;
-      for (int t = lane; t < ld; t += 32) cp_async8(rows + (k % kBandAhead) * ldm + t, B + i * ld + t);
+  const int per = (n + kBackRows - 1) / kBackRows, nb = per * nrhs;   // batches
+  if (threadIdx.x < 32) {
+    int k = 0;
+    for (int q = 0; q < nrhs; q++) {
+      const double *xr = x + (long)q * ldx + e0;
+      double z[NB];                          // rows i .. i - 32 NB + 1
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const int r = n - 1 - ((n - 1 - (lane + 32 * u)) & kMask);
+        z[u] = r >= 0 ? xr[r] : 0.0;
+      }
+#pragma unroll 1
+      for (int i0 = n - 1; i0 >= 0; i0 -= kBackRows, k++) {
+        const int st = k & (kBackStages - 1);
+        band_sync(1 + st, 64);
+        const double *Ls = rows + (size_t)st * kBackRows * ldm, *zs = zin + st * kBackRows;
+#pragma unroll
+        for (int t = 0; t < kBackRows; t++) {
+          const int i = i0 - t;
+          if (i < 0) break;
+          const double *Li = Ls + t * ldm;
+          const double zi = zs[t];
+          int kk[NB];
+          double lv[NB];
+#pragma unroll
+          for (int u = 0; u < NB; u++) {
+            kk[u] = (i - lane - 32 * u) & kMask;     // i minus the slot's row
+            lv[u] = Li[min(kk[u], b)];
+          }
+          const double xi = window_row<NB>(z, i);
+          const int reach = min(b, i);
+#pragma unroll
+          for (int u = 0; u < NB; u++) {
+            if (kk[u] >= 1 && kk[u] <= reach) z[u] = fma(-lv[u], xi, z[u]);
+            if (kk[u] == 0) z[u] = zi;               // row i's slot takes row i - 32 NB
+          }
+          if (lane == 0) xout[st * kBackRows + t] = xi;
+        }
+        __syncwarp();
+        band_arrive(5 + st, 64);
+      }
+    }
+    return;
+  }
+  // batch k: rows i0 .. i0 - kBackRows + 1 of right-hand side k / per
+  auto take = [&](int k) {
+    const int st = k & (kBackStages - 1), i0 = n - 1 - (k % per) * kBackRows;
+    band_sync(5 + st, 64);
+    if (lane < kBackRows && i0 - lane >= 0)
+      x[(long)(k / per) * ldx + e0 + i0 - lane] = xout[st * kBackRows + lane];
+  };
+  for (int k = 0; k < nb + kBackStages; k++) {
+    const int st = k & (kBackStages - 1);
+    if (k >= kBackStages) take(k - kBackStages);
+    if (k < nb) {
+      const int i0 = n - 1 - (k % per) * kBackRows;
+      for (int t = 0; t < kBackRows && i0 - t >= 0; t++)
+        for (int e = lane; e < ld; e += 32)
+          cp_async8(rows + ((size_t)st * kBackRows + t) * ldm + e, B + (long)(i0 - t) * ld + e);
+      if (lane < kBackRows && i0 - lane - kWin >= 0)
+        cp_async8(zin + st * kBackRows + lane, x + (long)(k / per) * ldx + e0 + i0 - lane - kWin);
     }
     cp_async_commit();
+    // batch k - 2 has arrived
+    cp_async_wait<2>();
+    __syncwarp();
+    if (k >= 2 && k - 2 < nb) band_arrive(1 + ((k - 2) & (kBackStages - 1)), 64);
   }
-  const bool in_smem = n <= zcap;
-  for (int r = 0; r < nrhs; r++) {
-    double *xr = x + (long)r * ldx + e0;
-    double *z = in_smem ? zs : xr;
-    if (in_smem) {
-      for (int i = lane; i < n; i += 32) zs[i] = xr[i];
-      __syncwarp();
-    }
-    for (int i = n - 1; i >= 0; i--) {
-      const long k = (long)r * n + (n - 1 - i);
-      cp_async_wait<kBandAhead - 1>();
-      __syncwarp();
-      const double *Li = rows + (k % kBandAhead) * ldm;
-      const double xi = z[i];
-      const int m = min(b, i);
-      for (int t = lane; t < m; t += 32) z[i - 1 - t] = fma(-Li[1 + t], xi, z[i - 1 - t]);
-      __syncwarp();
-      // this ring row takes the row of sweep step k + kBandAhead
-      const long kn = k + kBandAhead;
-      if (kn < T) {
-        const long in = n - 1 - kn % n;
-        for (int t = lane; t < ld; t += 32) cp_async8(rows + (k % kBandAhead) * ldm + t, B + in * ld + t);
-      }
-      cp_async_commit();
-    }
-    if (in_smem) {
-      __syncwarp();
-      for (int i = lane; i < n; i += 32) xr[i] = zs[i];
-      __syncwarp();
-    }
-  }
-  cp_async_wait<0>();
 }
 
 // Forward substitution and diagonal scaling on factors already in the band
@@ -324,36 +409,44 @@ __global__ void k_band_forward(BandSystem S, int nrhs, double *x, int ldx) {
   }
 }
 
+// The rows in use, kBandAhead fetched ahead, and two: the chain reads a fetched
+// row two hand-offs after the warp that waited for it
 int ring_rows(int bmax) {
   int R = 1;
-  while (R < bmax + 1 + kBandAhead) R <<= 1;
+  while (R < bmax + 1 + kBandAhead + 2) R <<= 1;
   return R;
+}
+
+// rows of a window in registers: the width, the pivot's row and kBandAhead
+// rows for the loads of the next ones to arrive
+int window_regs(int bmax) {
+  const int rows = bmax + 1 + kBandAhead;
+  return rows <= 32 ? 1 : rows <= 64 ? 2 : 4;
 }
 
 size_t factor_smem(int bmax) {
   const size_t ldm = bmax + 1, R = ring_rows(bmax);
-  return (R * ldm + R * kBandMaxRhs + 3 * ldm) * sizeof(double);
+  return (R * ldm + 8 * 32 * window_regs(bmax) + 2 * kBandAhead * kBandMaxRhs) * sizeof(double);
 }
 
 // trailing entries per worker for the widest band, rounded up to a kernel
 // instance
 int entries_per_worker(int bmax) {
-  const int tri = bmax * (bmax + 1) / 2;
+  const int tri = bmax * (bmax - 1) / 2;
   const int k = (tri + kBandWorkers - 1) / kBandWorkers;
-  for (int c : {3, 6, 9, 12, 16, 20, 24, 32})
+  for (int c : {1, 2, 3, 4, 5, 6, 8, 12, 16})
     if (k <= c) return c;
   return -1;
 }
 
-template <int K>
-void launch_factor(const BandSystem &S, int nrhs, double *x, int ldx, size_t smem, int R,
-                   cudaStream_t s, int *err) {
-  if (cudaFuncSetAttribute(k_band_factor_win<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess) {
-    *err = XG_ECUDA;
-    return;
-  }
-  k_band_factor_win<K><<<S.ncomp, kBandThreads, smem, s>>>(S, nrhs, x, ldx, R);
+template <int K, int NB>
+int launch_factor(const BandSystem &S, int nrhs, double *x, int ldx, cudaStream_t s) {
+  const size_t smem = factor_smem(S.bmax);
+  if (cudaFuncSetAttribute(k_band_factor<K, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess)
+    return XG_ECUDA;
+  k_band_factor<K, NB><<<S.ncomp, kBandThreads, smem, s>>>(S, nrhs, x, ldx, ring_rows(S.bmax));
+  return cudaGetLastError() == cudaSuccess ? 0 : XG_ECUDA;
 }
 
 }  // namespace
@@ -386,22 +479,21 @@ int band_factor_async(const BandSystem &S, cudaStream_t s, int nrhs, double *x, 
   if (S.ncomp == 0) return 0;
   if (nrhs < 0 || nrhs > kBandMaxRhs) return XG_EINVAL;
   if (cudaMemsetAsync(S.flags, 0, 4 * sizeof(int), s) != cudaSuccess) return XG_ECUDA;
-  const size_t smem = factor_smem(S.bmax);
-  const int R = ring_rows(S.bmax);
-  int err = 0;
+  // widths up to 23 take one register of rows and at most two entries a
+  // worker, up to 55 two and at most eight, the rest (up to 77) four
   switch (entries_per_worker(S.bmax)) {
-    case 3: launch_factor<3>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 6: launch_factor<6>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 9: launch_factor<9>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 12: launch_factor<12>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 16: launch_factor<16>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 20: launch_factor<20>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 24: launch_factor<24>(S, nrhs, x, ldx, smem, R, s, &err); break;
-    case 32: launch_factor<32>(S, nrhs, x, ldx, smem, R, s, &err); break;
+    case 1: return launch_factor<1, 1>(S, nrhs, x, ldx, s);
+    case 2: return window_regs(S.bmax) == 1 ? launch_factor<2, 1>(S, nrhs, x, ldx, s)
+                                            : launch_factor<2, 2>(S, nrhs, x, ldx, s);
+    case 3: return launch_factor<3, 2>(S, nrhs, x, ldx, s);
+    case 4: return launch_factor<4, 2>(S, nrhs, x, ldx, s);
+    case 5: return launch_factor<5, 2>(S, nrhs, x, ldx, s);
+    case 6: return launch_factor<6, 2>(S, nrhs, x, ldx, s);
+    case 8: return launch_factor<8, 2>(S, nrhs, x, ldx, s);
+    case 12: return launch_factor<12, 4>(S, nrhs, x, ldx, s);
+    case 16: return launch_factor<16, 4>(S, nrhs, x, ldx, s);
     default: return XG_EINVAL;
   }
-  if (err || cudaGetLastError() != cudaSuccess) return XG_ECUDA;
-  return 0;
 }
 
 int band_factor(const BandSystem &S, cudaStream_t s, int *bad_eq, int nrhs, double *x, int ldx) {
@@ -422,14 +514,12 @@ int band_solve(const BandSystem &S, int nrhs, double *x, int ldx, cudaStream_t s
     const int warps = 4;
     k_band_forward<<<(S.ncomp + warps - 1) / warps, 32 * warps, 0, s>>>(S, nrhs, x, ldx);
   }
-  // z in shared memory for parts of up to 2,048 equations
-  const int zcap = S.nmax <= 2048 ? S.nmax : 0;
-  const size_t smem = (size_t)kBackWarps * (kBandAhead * (S.bmax + 1) + zcap) * sizeof(double);
-  if (cudaFuncSetAttribute(k_band_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return XG_ECUDA;
-  k_band_back<<<(S.ncomp + kBackWarps - 1) / kBackWarps, 32 * kBackWarps, smem, s>>>(S, nrhs, x,
-                                                                                      ldx, zcap);
+  const size_t smem = back_smem(S.bmax);
+  switch (window_regs(S.bmax)) {
+    case 1: k_band_back<1><<<S.ncomp, 64, smem, s>>>(S, nrhs, x, ldx); break;
+    case 2: k_band_back<2><<<S.ncomp, 64, smem, s>>>(S, nrhs, x, ldx); break;
+    default: k_band_back<4><<<S.ncomp, 64, smem, s>>>(S, nrhs, x, ldx); break;
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : XG_ECUDA;
 }
 
