@@ -99,7 +99,7 @@ struct PcgSystem {
                           // (padded to 6 x 6) when kb is 0
   // work vectors [n]
   double *r, *z, *p, *q;
-  double *partials;       // [4*pcg_max_blocks() + 8] (3*... + 8 without the node-block copy)
+  double *partials;       // [pcg_partial_doubles()] (3*pcg_max_blocks() + 8 without the copy)
   unsigned int *barrier;  // [2] grid barrier state
   int *flags;             // [4] status words
   double *scalars;        // [8]
@@ -109,7 +109,7 @@ struct PcgSystem {
   // nb_cap blocks; the rows of longer node rows in chunks of CSR entries, a
   // warp each; nb_vals null: every row is read from the CSR arrays warp per
   // row.  The block SpMV computes in float-float (each value and each entry
-  // of p split into two single-precision numbers, xg_ff.h) on the
+  // of z split into two single-precision numbers, xg_ff.h) on the
   // single-precision pipes; node rows with a value outside the split's range
   // stay in FP64.
   int kb;                 // block order: 2, 3 or 6 (the largest diagonal block), 0: no copy
@@ -117,15 +117,18 @@ struct PcgSystem {
   const int *nb_cols;     // [nb_off[last]] column node of each block
   const int *nb_len;      // [nblk] blocks of each node row
   const int *nb_pos;      // [nnz] slot of each CSR entry in nb_vals (-1: a long node row's)
-  float2 *nb_vals;        // [nb_off[last]*kb*kb] (hi, lo), packed by pcg_factor_blocks
+  float2 *nb_vals;        // [block_ell_pairs] records of a block's (hi, lo) values and its
+                          // column nodes, packed by pcg_factor_blocks
   unsigned char *blk_ff;  // [nblk] 1: the node row's values lie in the split's range
-  float2 *p2;             // [nblk*(kb == 3 ? 4 : kb)] p split, node-major, padding zero
+  float2 *p2;             // [nblk*(kb == 3 ? 4 : kb)] z split, node-major, padding zero
   int nb_cap;
   int nlong, nchunks;     // long rows, their chunks
   const int *chunk_row;   // [nchunks] row of each chunk
   const int *chunk_beg;   // [nchunks] first CSR entry of each chunk
   const int *long_chunk0; // [nlong+1] chunk range of each long row
-  double *chunk_part;     // [nchunks] partial sums
+  int nlongn;             // long node rows, their nodes and first long rows
+  const int *long_node, *long_row0;
+  double *chunk_part;     // [4 nchunks] partial sums
 };
 // Factor the diagonal blocks (and pack the node-block values when present)
 // after the matrix values changed.
@@ -139,13 +142,14 @@ struct BlockEll {
   int kb = 0;
   std::vector<long> off;
   std::vector<int> cols, len, pos;
-  std::vector<int> chunk_row, chunk_beg, long_chunk0;
+  std::vector<int> chunk_row, chunk_beg, long_chunk0, long_node, long_row0;
 };
 int block_ell_layout(int n, const int *rowptr, const int *colidx, int nblk, const int *blk_start,
                      int cap, BlockEll &h);
 // Device bytes of the copy (columns, values, positions, offsets, per-node
 // arrays and p2).
 size_t block_ell_bytes(const BlockEll &h, int nblk);
+size_t block_ell_pairs(const BlockEll &h);
 // Solve A x = b (device vectors).  x holds the initial guess (usually 0).
 // Returns 0 when converged, XG_ESOLVE on breakdown, maxit or a barrier timeout.
 // rows_per_block: the grid gets one block per that many rows (capped by
@@ -153,6 +157,7 @@ size_t block_ell_bytes(const BlockEll &h, int nblk);
 int pcg_solve(const PcgSystem &S, const double *b, double *x, double rtol, int maxit,
               int *iters, double *relres, cudaStream_t s, int rows_per_block = 0);
 int pcg_max_blocks();
+size_t pcg_partial_doubles();
 
 // Skyline LDL' without pivoting on 32 x 32 tiles (xg_profile.cu)
 struct ProfileSystem {

@@ -58,7 +58,8 @@ struct xg_linsoe {
   // device copies, set up at the first solve
   bool ready = false;
   cudaStream_t stream = nullptr;
-  DevArray<int> rp, ci, bs, chunk_row, chunk_beg, long_chunk0, nb_cols, nb_len, nb_pos, flags;
+  DevArray<int> rp, ci, bs, chunk_row, chunk_beg, long_chunk0, long_node, long_row0;
+  DevArray<int> nb_cols, nb_len, nb_pos, flags;
   DevArray<long> nb_off;
   DevArray<unsigned int> barrier;
   DevArray<double> vals, b, x, binv, r, z, p, q, partials, scalars, chunk_part;
@@ -115,11 +116,11 @@ struct xg_linsoe {
     e |= vals.alloc(std::max<size_t>(nnz, 1)) | b.alloc(nv) | x.alloc(nv);
     e |= binv.alloc((size_t)std::max(nblk, 1) * 36);
     e |= r.alloc(nv) | z.alloc(nv) | p.alloc(nv) | q.alloc(nv);
-    e |= partials.alloc(4 * (size_t)xg::pcg_max_blocks() + 8);
+    e |= partials.alloc(xg::pcg_partial_doubles());
     e |= scalars.alloc(8) | barrier.alloc(2) | flags.alloc(4);
     size_t nvals = 0, np2 = 0;
     if (h.kb) {
-      nvals = std::max<size_t>((size_t)h.off.back() * h.kb * h.kb, 1);
+      nvals = std::max<size_t>(xg::block_ell_pairs(h), 1);
       np2 = (size_t)nblk * (h.kb == 3 ? 4 : h.kb);
       e |= nb_off.upload(h.off.data(), h.off.size(), stream);
       e |= nb_cols.upload(h.cols.data(), h.cols.size(), stream);
@@ -129,7 +130,9 @@ struct xg_linsoe {
       e |= chunk_row.upload(h.chunk_row.data(), h.chunk_row.size(), stream);
       e |= chunk_beg.upload(h.chunk_beg.data(), h.chunk_beg.size(), stream);
       e |= long_chunk0.upload(h.long_chunk0.data(), h.long_chunk0.size(), stream);
-      e |= chunk_part.alloc(std::max<size_t>(h.chunk_row.size(), 1));
+      e |= long_node.upload(h.long_node.data(), h.long_node.size(), stream);
+      e |= long_row0.upload(h.long_row0.data(), h.long_row0.size(), stream);
+      e |= chunk_part.alloc(std::max<size_t>(4 * h.chunk_row.size(), 1));
     }
     if (e) return lfail(XG_ENOMEM, "xg_linsoe: device allocation failed");
     if (h.kb && (cudaMemsetAsync(nb_vals.p, 0, nvals * sizeof(float2), stream) != cudaSuccess ||
@@ -165,6 +168,9 @@ struct xg_linsoe {
       S.chunk_row = chunk_row.p;
       S.chunk_beg = chunk_beg.p;
       S.long_chunk0 = long_chunk0.p;
+      S.nlongn = (int)h.long_node.size();
+      S.long_node = long_node.p;
+      S.long_row0 = long_row0.p;
       S.chunk_part = chunk_part.p;
     }
     if (cudaStreamSynchronize(stream) != cudaSuccess)

@@ -243,7 +243,7 @@ struct xg_model {
   DBuf<unsigned char> d_blk_ff;
   DBuf<double> d_geo;   // bricks: per-point shape-function gradients and Jacobian determinant
   DBuf<float2> d_geo2;  // bricks: the gradients split into float pairs (float-float tangent)
-  DBuf<int> d_chunk_row, d_chunk_beg, d_long_chunk0;
+  DBuf<int> d_chunk_row, d_chunk_beg, d_long_chunk0, d_long_node, d_long_row0;
   bool blocks_tried = false;
   long long pcg_blocks = 0;   // node-pair blocks of the PCG's copy
   int ensure_pcg_blocks();
@@ -814,7 +814,7 @@ int xg_model::upload(const HostGather &gk_h, const HostGather &gr_h) {
   RET(d_binv.alloc((size_t)std::max(nblk, 1) * 36));
   const size_t nv = neq > 0 ? neq : 1;
   RET(d_r.alloc(nv)); RET(d_z.alloc(nv)); RET(d_p.alloc(nv)); RET(d_q.alloc(nv));
-  RET(d_pcg_part.alloc(4 * (size_t)pcg_max_blocks() + 8));
+  RET(d_pcg_part.alloc(pcg_partial_doubles()));
   RET(d_scalars.alloc(8));
   RET(d_barrier.alloc(2));
   RET(d_flags.alloc(4));
@@ -1598,7 +1598,7 @@ int xg_model::ensure_pcg_blocks() {
   RET(d_nb_cols.upload(h.cols.data(), h.cols.size(), stream));
   RET(d_nb_len.upload(h.len.data(), h.len.size(), stream));
   RET(d_nb_pos.upload(h.pos.data(), h.pos.size(), stream));
-  RET(d_nb_vals.alloc(std::max<size_t>((size_t)h.off.back() * h.kb * h.kb, 1)));
+  RET(d_nb_vals.alloc(std::max<size_t>(block_ell_pairs(h), 1)));
   CK(cudaMemsetAsync(d_nb_vals.p, 0, d_nb_vals.n * sizeof(float2), stream));
   RET(d_p2.alloc((size_t)nblk * ks));
   CK(cudaMemsetAsync(d_p2.p, 0, d_p2.n * sizeof(float2), stream));
@@ -1607,7 +1607,12 @@ int xg_model::ensure_pcg_blocks() {
   RET(d_chunk_row.upload(h.chunk_row.data(), h.chunk_row.size(), stream));
   RET(d_chunk_beg.upload(h.chunk_beg.data(), h.chunk_beg.size(), stream));
   RET(d_long_chunk0.upload(h.long_chunk0.data(), h.long_chunk0.size(), stream));
-  RET(d_chunk_part.alloc(std::max(nch, 1)));
+  RET(d_chunk_part.alloc(std::max<size_t>(4 * (size_t)nch, 1)));
+  RET(d_long_node.upload(h.long_node.data(), h.long_node.size(), stream));
+  RET(d_long_row0.upload(h.long_row0.data(), h.long_row0.size(), stream));
+  pcg.nlongn = (int)h.long_node.size();
+  pcg.long_node = d_long_node.p;
+  pcg.long_row0 = d_long_row0.p;
   pcg.kb = h.kb;
   pcg_blocks = 0;
   for (int i = 0; i < nblk; i++)
