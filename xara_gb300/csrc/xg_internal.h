@@ -188,8 +188,12 @@ struct ProfileSystem {
   int *cplw, *cpl, *cplq;
   // columns published by the factorisation: [nt][column][row] of L_JJ (the
   // reciprocal pivot on the diagonal), then [nt][column][P rows, L rows] of
-  // panel (J+1, J)
-  double *lstream, *wlstream;
+  // panel (J+1, J), then the same of panel (J+2, J)
+  double *lstream, *wlstream, *w2stream;
+  // tile rows kept by row blocks: [nt] first column, [nt] the slot's next row (nt:
+  // none), [nslots] a slot's first row
+  const int *own_first, *next_row, *slot_row;
+  int nslots;
   // right-hand sides whose forward sweep runs inside the factorisation
   // (fwd_nrhs 0: none)
   int fwd_nrhs;
@@ -198,8 +202,10 @@ struct ProfileSystem {
 };
 int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &ftile, int &nt,
                  int &W);
-void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks,
-                   std::vector<int> &npairs);
+void profile_rows(int nt, const std::vector<int> &ftile, std::vector<int> &first,
+                  std::vector<int> &next, std::vector<int> &slot_row);
+void profile_tasks(int nt, int W, const std::vector<int> &ftile, const std::vector<int> &first,
+                   std::vector<int> &tasks, std::vector<int> &npairs);
 size_t profile_tile_doubles(int nt, int W);
 size_t profile_digit_bytes(int W);
 int profile_tile_edge();
@@ -254,7 +260,7 @@ class ProfileSolver {
   ProfileSystem S_{};
   int fwd_nrhs_ = 0;         // right-hand sides factor_forward swept
   bool ready_ = false;
-  Buf<int> ftile_, counters_, tasks_, npairs_;
+  Buf<int> ftile_, counters_, tasks_, npairs_, rows_;
   Buf<unsigned char> dig_;
   Buf<double> L_, invD_, piv_, Winv_, F_, G_, E_, H_, Q_, R_, sweep_, stream_;
 };

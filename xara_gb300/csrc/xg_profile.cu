@@ -36,19 +36,24 @@
 // none.  (The idea of error-free digit products: K. Ozaki, T. Ogita, S. Oishi
 // and S. M. Rump, Numer. Algorithms 59, 2012.)
 //
-// Who runs what.  One persistent cooperative launch, a block per SM.  Tile
-// J's elimination (block `diag` J mod 3), the panel (J+1, J) (block `panel` J
-// mod 2) and that panel's update of diagonal tile J+1 (the next diag block)
-// run as a stream: the elimination publishes every column of L_JJ as it is
-// formed, the panel block solves its column with it and publishes P and L of
-// that column, the next diag block takes the column off its tile, so the next
-// tile is ready two hand-offs after the last pivot instead of after a solve
-// and a product.  These are FP64 with the operands of the plain order (an
-// explicit inverse of L_JJ would let the panels be products, but costs two
-// digits: energy norm error 7e-13 against 4e-15 on a 64 x 16 quad block).
-// The other blocks take the remaining panels (the same streamed solve), the
-// tile pairs and the substitutions' matrices from a list in look-ahead
-// order; their ninth warp draws the next task and waits for its operands
+// Who runs what.  One persistent cooperative launch, a block per SM.  What the
+// next tile column waits for runs as a stream, in FP64 with the operands of the
+// plain order (an explicit inverse of L_JJ would let the panels be products, but
+// costs two digits: energy norm error 7e-13 against 4e-15 on a 64 x 16 quad
+// block).  Tile J's elimination (block `diag` J mod 3) publishes every column of
+// L_JJ as it is formed.  A tile row I belongs to two row blocks, 16 rows each,
+// from its first column to its last: column by column they
+// solve (I, J) and take P_IJ L_J+1,J' off tile (I, J+1), which they keep in
+// registers, and row J+1's publish their columns of P and L for that and for the
+// next diag block, which takes them off tile J+1.  So the next diagonal tile and
+// every row's next panel are ready two hand-offs after the last pivot.  With the
+// panels and those products from the list each row took solve, digits, product
+// and three flags a column, 14.8 us however fast the eliminations (9) were.  A
+// tile column takes 12.5 us now on a 64 x 16 quad block (63 of them, 15.4 before)
+// and 13.7 on a 10 x 10 x 20 frame (454, 15.4): the elimination and 3 us from its
+// last column to the next one's first, of which the two hand-offs are half.
+// The other blocks take the other panels, the other tile pairs and the
+// substitutions' matrices from a list in look-ahead order; their ninth warp draws the next task and waits for its operands
 // (bounded by the global timer) while the eight others compute.  Every
 // dependency sits earlier in the list or in the stream, and the digits live
 // in a ring of kRing tile columns (a column's slots are refilled when its
@@ -82,7 +87,10 @@ constexpr int kOpBytes = kDigitBytes + kT * 4;
 // ring slot of a panel tile: P, then L
 constexpr int kSlotBytes = 2 * kOpBytes;
 constexpr int kRing = 8;
-constexpr int kDiagBlocks = 3, kPanelBlocks = 2;   // the stream's own blocks
+constexpr int kDiagBlocks = 3;
+// the stream's blocks: four warps that poll, four for the row blocks' digits
+constexpr int kPollThreads = 128, kDigitThreads = 128;
+constexpr int kBlockThreads = kComputeThreads + kPollThreads + kDigitThreads;
 constexpr int kBadExp = 1 << 28;       // the exponent of a row with an infinity or a NaN
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -104,7 +112,7 @@ __global__ void k_prof_prepare(ProfileSystem S, size_t ncount, size_t nsweep) {
   const size_t gthreads = (size_t)gridDim.x * blockDim.x;
   const double none = __longlong_as_double((long long)0xFFFFFFFFFFFFFFFFull);
   for (size_t k = gtid; k < ncount; k += gthreads) S.flags[k] = 0;
-  for (size_t k = gtid; k < 3 * (size_t)S.nt * kTT; k += gthreads) S.lstream[k] = none;
+  for (size_t k = gtid; k < 5 * (size_t)S.nt * kTT; k += gthreads) S.lstream[k] = none;
   for (size_t k = gtid; k < nsweep; k += gthreads) S.sweep[k] = none;
   const int lane = threadIdx.x & 31;
   for (int i = (int)(gtid >> 5); i < S.nt * kT; i += (int)(gthreads >> 5)) {
@@ -153,6 +161,17 @@ __device__ __noinline__ bool wait_slow(const int *p, int target, volatile int *f
 }
 __device__ __forceinline__ bool wait_geq(const int *p, int target, volatile int *flags) {
   return *(const volatile int *)p >= target || wait_slow(p, target, flags);
+}
+
+// The same with the order of the loads behind it (half the time of a fence).
+__device__ __forceinline__ bool wait_acquire(const int *p, int target, volatile int *flags) {
+  for (int k = 0;; k++) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    if (v >= target) return true;
+    if (k == 0) continue;
+    if (!wait_slow(p, target, flags)) return false;
+  }
 }
 
 // Published values: a scratch vector is filled with kUnset beforehand (a NaN
@@ -217,6 +236,8 @@ __device__ __forceinline__ void publish(double *p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
+// the computing and the polling warps
+__device__ __forceinline__ void bsync() { named_sync(11, kComputeThreads + kPollThreads); }
 // the eight computing warps
 __device__ __forceinline__ void csync() { named_sync(9, kComputeThreads); }
 
@@ -475,14 +496,37 @@ __device__ void eliminate_tile(FactorSmem &sm, int warp, int lane, const TrailEn
   }
 }
 
+// Row r of a solved panel (I = J+o, J), row rs of the columns W of P and L in
+// shared memory: L to the tile, P and L as digits to the ring slot; the eight
+// threads q of a row adjacent.
+template <int N>
+__device__ __forceinline__ void panel_store(const ProfileSystem &S, const double (*W)[N],
+                                            const double (*L)[N], const double *inv, int r, int rs,
+                                            int q, int o, int J) {
+  double p[4], l[4];
+  int t[4], nt[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    p[i] = W[4 * q + i][rs];
+    l[i] = L[4 * q + i][rs];
+    nt[i] = half_exp(inv[4 * q + i]);
+    t[i] = -nt[i];
+  }
+  double2 *tile = reinterpret_cast<double2 *>(tile_at(S, J + o, o) + r * kT + 4 * q);
+  tile[0] = make_double2(l[0], l[1]);
+  tile[1] = make_double2(l[2], l[3]);
+  unsigned char *slot = dig_slot(S, J, o);
+  slice_row4(p, t, r, q, slot);
+  slice_row4(l, nt, r, q, slot + kOpBytes);
+}
+
 // Phase B on tile (I, J): P L_JJ' = A, L = P D^-1, column by column as L_JJ
 // is published.  Lane = row; warp w of the eight computing ones holds columns
 // w, w+8, w+16, w+24 in registers, so that a column's FMAs fill whole warps
 // (496 in all: 9,400 cycles of the FP64 unit, below the elimination's own
 // time); the warp whose column is final hands it to the others through shared
 // memory.  The ninth warp polls the published columns (panel_poll), a column
-// ahead of the others; one barrier a column.  With wl, P and L of each column
-// are published for the block that holds diagonal tile I.  Afterwards L goes
+// ahead of the others; one barrier a column.  Afterwards L goes
 // to the tile and both, as digits, to the ring slot.
 __device__ void panel_poll(const ProfileSystem &S, FactorSmem &sm, int J, int lane,
                            volatile int *flags) {
@@ -498,8 +542,7 @@ __device__ void panel_poll(const ProfileSystem &S, FactorSmem &sm, int J, int la
     named_sync(10, kFactorThreads);
   }
 }
-__device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J, int tid,
-                           double *wl) {
+__device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J, int tid) {
   const int r = tid >> 3, q = tid & 7, o = I - J, w = tid >> 5, lane = tid & 31;
   double *tile = tile_at(S, I, o) + r * kT + 4 * q;
   double x[4];
@@ -509,10 +552,7 @@ __device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J,
   csync();
 #pragma unroll
   for (int j = 0; j < 4; j++) x[j] = sm.A[lane][8 * j + w];
-  if (w == 0) {
-    sm.W[0][lane] = x[0];
-    if (wl) publish(wl + lane, x[0]);
-  }
+  if (w == 0) sm.W[0][lane] = x[0];
 #pragma unroll
   for (int jc = 0; jc < 4; jc++) {
     for (int c8 = 0; c8 < 8; c8++) {
@@ -525,35 +565,18 @@ __device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J,
         const int s = 8 * j + w;
         if (j >= jc && s > c) {
           x[j] = fma(-wc, lc[s], x[j]);
-          if (s == c + 1) {
-            sm.W[s][lane] = x[j];
-            if (wl) publish(wl + s * 2 * kT + lane, x[j]);
-          }
+          if (s == c + 1) sm.W[s][lane] = x[j];
         }
       }
       if (w == c8) {      // column c is this warp's: scale it
         const double inv = lc[c], v = x[jc] * inv;
         sm.L[c][lane] = v;
         if (lane == 0) sm.inv[c] = inv;
-        if (wl) publish(wl + c * 2 * kT + kT + lane, v);
       }
     }
   }
   csync();
-  double p[4], l[4];
-  int t[4], nt[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    p[i] = sm.W[4 * q + i][r];
-    l[i] = sm.L[4 * q + i][r];
-    nt[i] = half_exp(sm.inv[4 * q + i]);
-    t[i] = -nt[i];
-  }
-  reinterpret_cast<double2 *>(tile)[0] = make_double2(l[0], l[1]);
-  reinterpret_cast<double2 *>(tile)[1] = make_double2(l[2], l[3]);
-  unsigned char *slot = dig_slot(S, J, o);
-  slice_row4(p, t, r, q, slot);
-  slice_row4(l, nt, r, q, slot + kOpBytes);
+  panel_store(S, sm.W, sm.L, sm.inv, r, r, q, o, J);
 }
 
 // Phase C on pair (I = J+a, K = J+b), b <= a: A_IK -= P_IJ L_KJ'.  On a
@@ -665,6 +688,15 @@ __device__ void second_coupling_task(const ProfileSystem &S, FactorSmem &sm, int
 // Dependencies of a list task (type, I, K, J): every update of its tile from
 // earlier columns (the count of columns J' < J both tile rows reach), and the
 // diagonal / panel tiles it reads.
+// how often tile (I, J) is reported done: a panel of the row blocks by eight
+// warps
+__device__ __forceinline__ int done_count(const ProfileSystem &S, int I, int J) {
+  return I > J && J >= S.own_first[I] ? 2 * kDigitThreads / 32 : 1;
+}
+__device__ __forceinline__ bool wait_done(const ProfileSystem &S, int I, int J,
+                                          volatile int *flags) {
+  return wait_geq(S.done + slot_of(S, I, I - J), done_count(S, I, J), flags);
+}
 enum { kPanel = 1, kPair = 2, kInverse = 5, kCouple = 6, kForward = 7, kCouple2 = 8 };
 __device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
   const int type = t.x, I = t.y, K = t.z, J = t.w;
@@ -672,14 +704,13 @@ __device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
     return (J < kRing || wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags)) &&
            wait_geq(S.upd + slot_of(S, I, I - J), J - max(S.ftile[I], S.ftile[J]), flags);
   if (type == kPair)
-    return wait_geq(S.done + slot_of(S, I, I - J), 1, flags) &&
-           wait_geq(S.done + slot_of(S, K, K - J), 1, flags) &&
+    return wait_done(S, I, J, flags) && wait_done(S, K, J, flags) &&
            wait_geq(S.upd + slot_of(S, I, I - K), J - max(S.ftile[I], S.ftile[K]), flags);
-  if (type == kInverse) return wait_geq(S.done + slot_of(S, J, 0), 1, flags);
+  if (type == kInverse) return wait_done(S, J, J, flags);
   if (type == kCouple) {
     int Ic, o;
     if (!wait_geq(S.cplw + J, 1, flags)) return false;
-    return !coupling_tile(S, J, K, &Ic, &o) || wait_geq(S.done + slot_of(S, Ic, o), 1, flags);
+    return !coupling_tile(S, J, K, &Ic, &o) || wait_done(S, Ic, Ic - o, flags);
   }
   if (type == kCouple2) {
     const int O = K == 0 ? J - 1 : J + 1;    // the neighbour's F or G
@@ -692,7 +723,7 @@ __device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
   if (!wait_geq(S.cplq + J, 1, flags)) return false;
   const int ohi = min(S.W, J - S.ftile[J]);
   for (int o = 3; o <= ohi; o++)
-    if (!wait_geq(S.done + slot_of(S, J, o), 1, flags)) return false;
+    if (!wait_done(S, J, J - o, flags)) return false;
   return true;
 }
 
@@ -794,10 +825,11 @@ __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
 }
 
 // Diagonal tiles J = first, first + kDiagBlocks, ...: the tile, updated by
-// the columns before J-1, loses panel (J, J-1) column by column as it is
-// published, then it is factored.  The packed lower triangle sits in
+// the columns before J-2, loses panels (J, J-2) and (J, J-1) column by column as
+// they are published, then it is factored.  The packed lower triangle sits in
 // registers meanwhile (rows 31-s and s-1 in the lanes of slot s, 17 slots on
-// eight warps); the ninth warp polls.
+// eight warps); four warps poll, a column in four each, since a look at a published
+// value takes longer than a column.
 constexpr int kSlots = 17;
 __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, volatile int *flags) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -806,32 +838,33 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
   if (tid == kComputeThreads) sm.fail = 0;
   for (int J = first; J < S.nt; J += kDiagBlocks) {
     const bool fed = J > 0 && S.ftile[J] < J;
-    if (warp == 8 && lane == 0) {
-      if (fed && !wait_geq(S.upd + slot_of(S, J, 0), J - 1 - S.ftile[J], flags)) sm.fail = 1;
-      __threadfence();
-    }
-    __syncthreads();
-    if (sm.fail) return;
+    const bool fed2 = J > 1 && S.ftile[J] < J - 1;
     const double *tile = tile_at(S, J, 0);
     if (fed) {
-      if (warp == 8) {
-        const double *wl = S.wlstream + (size_t)(J - 1) * 2 * kTT;
-        double a = ld_relaxed(wl + lane), b = ld_relaxed(wl + kT + lane);
-        for (int c = 0; c < kT; c++) {
-          // L is published after P: once it is there, P is a load away
-          if (unset(b)) {
-            b = await_column(wl + c * 2 * kT + kT + lane, flags);
-            if (unset(a)) a = ld_relaxed(wl + c * 2 * kT + lane);
+      if (warp >= 8) {
+        const int k = warp - 8;
+        for (int back = fed2 ? 2 : 1; back >= 1; back--) {
+          const double *wl = (back == 2 ? S.w2stream : S.wlstream) + (size_t)(J - back) * 2 * kTT + lane;
+          double a = ld_relaxed(wl + k * 2 * kT), b = ld_relaxed(wl + k * 2 * kT + kT);
+          for (int c = k; c < kT; c += 4) {
+            // L is published after P: once it is there, P is a load away
+            if (unset(b)) {
+              b = await_column(wl + c * 2 * kT + kT, flags);
+              if (unset(a)) a = ld_relaxed(wl + c * 2 * kT);
+            }
+            if (unset(a)) a = await_column(wl + c * 2 * kT, flags);
+            sm.W[c][lane] = a;
+            sm.L[c][lane] = b;
+            if (back == 1 && c == 0 && lane == 0 &&
+                !wait_acquire(S.upd + slot_of(S, J, 0), max(J - 2 - S.ftile[J], 0), flags))
+              sm.fail = 1;
+            if (c + 4 < kT) {
+              a = ld_relaxed(wl + (c + 4) * 2 * kT);
+              b = ld_relaxed(wl + (c + 4) * 2 * kT + kT);
+            }
+            __syncwarp();
+            named_sync(12 + k, kFactorThreads);
           }
-          if (unset(a)) a = await_column(wl + c * 2 * kT + lane, flags);
-          sm.W[c][lane] = a;
-          sm.L[c][lane] = b;
-          if (c + 1 < kT) {
-            a = ld_relaxed(wl + (c + 1) * 2 * kT + lane);
-            b = ld_relaxed(wl + (c + 1) * 2 * kT + kT + lane);
-          }
-          __syncwarp();
-          named_sync(10, kFactorThreads);
         }
       } else {
         int rw[3], kk[3];
@@ -845,16 +878,22 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
             if (lane < kT - s) { rw[u] = kT - 1 - s; kk[u] = lane; }
             else if (s < kSlots - 1) { rw[u] = s - 1; kk[u] = lane - (kT - s); }
           }
-          m[u] = rw[u] >= 0 ? __ldcg(tile + rw[u] * kT + kk[u]) : 0.0;
-          acc[u] = 0.0;
+          m[u] = acc[u] = 0.0;
         }
-        // the products are summed on their own and taken off once, as the
+        // the tile itself comes in when its other updates have (they are late
+        // ones); the products are summed on their own and taken off once, as the
         // tile pairs' are: one rounding at the size of the tile's entry
-        for (int c = 0; c < kT; c++) {
-          named_sync(10, kFactorThreads);
+        for (int k = fed2 ? 0 : kT; k < 2 * kT; k++) {
+          const int c = k & (kT - 1);
+          named_sync(12 + (c & 3), kFactorThreads);
 #pragma unroll
           for (int u = 0; u < 3; u++)
             if (rw[u] >= 0) acc[u] = fma(sm.W[c][rw[u]], sm.L[c][kk[u]], acc[u]);
+          if (k == kT) {
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+              if (rw[u] >= 0) m[u] = __ldcg(tile + rw[u] * kT + kk[u]);
+          }
         }
 #pragma unroll
         for (int u = 0; u < 3; u++)
@@ -863,9 +902,10 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
     } else if (tid < kComputeThreads) {
       for (int k = tid; k < kTT; k += kComputeThreads) sm.A[k >> 5][k & 31] = __ldcg(tile + k);
     }
-    __syncthreads();
+    bsync();
+    if (sm.fail) return;
     if (warp < 8) eliminate_tile(sm, warp, lane, te, S.lstream + (size_t)J * kTT);
-    __syncthreads();
+    bsync();
     if (tid < kT) {
       const int eq = J * kT + tid;
       const double d = sm.L[tid][tid];
@@ -893,7 +933,7 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
       g[0] = make_double2(v[0], v[1]);
       g[1] = make_double2(v[2], v[3]);
     }
-    __syncthreads();
+    bsync();
     if (sm.fail) return;
     if (tid == 0) {
       __threadfence();
@@ -902,26 +942,202 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
   }
 }
 
-// Panels (J+1, J) for J = first, first + kPanelBlocks, ...
-__device__ void panel_block(const ProfileSystem &S, FactorSmem &sm, int first,
-                            volatile int *flags) {
-  const int tid = threadIdx.x;
-  for (int J = first; J + 1 < S.nt; J += kPanelBlocks) {
-    if (S.ftile[J + 1] > J) continue;
-    if (tid == 0) {
-      sm.fail = !((J < kRing || wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags)) &&
-                  wait_geq(S.upd + slot_of(S, J + 1, 1), J - max(S.ftile[J + 1], S.ftile[J]),
-                           flags));
+// Rows 16 half .. 16 half + 15 of the tile rows I of a slot: for every column J
+// from S.own_first[I] to I-1 the solve of (I, J), P L_JJ' = A and L = P D^-1, and, kLag
+// columns behind it, the update of tile (I, J+1) with the published columns of
+// L_J+1,J; the next solve starts from these registers.
+//
+// Warp 0 carries the chain of the panel's columns (lane = row): it takes the two
+// newest columns off column t, publishes it and scales it.  Warps 1-7 apply a
+// column to those three and more behind it and to tile (I, J+1), a row and a
+// column parity a lane, column pairs w-1, w+6, w+13; so a column is not as long as
+// their turns at the FP64 unit (33 warp operations at first, 17 at last, 475
+// cycles on average) and the chain's latency together: 690 cycles with all eight
+// warps in step, where the elimination takes 540.  Four warps poll the two streams,
+// a column in four each: a look at a published value takes some 900 cycles (eight
+// slots, so that a warp fills the next one while its last is read).  Four more
+// write the finished panel and its digits while the others are at the next.
+// Barriers: 1-4 a column is polled (to the chain), 5-7 the chain has it (to the
+// others), 8-10 the others have applied it, 12-13 a panel's buffer is full, 14-15
+// it is free.
+constexpr int kLag = 4;                // a multiple of the four polling warps
+struct RowSmem {
+  double W[2][kT][17], L[2][kT][17];   // P and L by columns, two panels
+  double R[kT][17];                    // columns with all but the two newest applied
+  double inv[2][kT];
+  double Lc[8][kT], Ln[8][kT];         // the streams' columns being applied
+  int fail;
+};
+static_assert(sizeof(RowSmem) <= kFactorSmem, "");
+__device__ void row_digits(const ProfileSystem &S, RowSmem &sm, int slot, int half,
+                           volatile int *flags) {
+  const int tid = threadIdx.x - kComputeThreads - kPollThreads, lane = tid & 31;
+  int n = 0;
+  for (int I = S.slot_row[slot]; I < S.nt; I = S.next_row[I])
+    for (int J = S.own_first[I]; J < I; J++, n++) {
+      const int buf = n & 1;
+      named_sync(12 + buf, 32 + kDigitThreads);
+      if (sm.fail) return;
+      // the ring slot's last user has gone (a failed wait raises flags[0])
+      if (lane == 0 && J >= kRing) {
+        wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags);
+        __threadfence();
+      }
+      __syncwarp();
+      panel_store(S, sm.W[buf], sm.L[buf], sm.inv[buf], 16 * half + (tid >> 3), tid >> 3, tid & 7,
+                  I - J, J);
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence();
+        atomicAdd(S.done + slot_of(S, I, I - J), 1);
+      }
+      named_arrive(14 + buf, 32 + kDigitThreads);
+    }
+}
+
+__device__ void row_block(const ProfileSystem &S, RowSmem &sm, int slot, int half,
+                          volatile int *flags) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  if (tid == 0) sm.fail = 0;
+  __syncthreads();
+  if (w >= 12) {
+    row_digits(S, sm, slot, half, flags);
+    return;
+  }
+  const int r16 = lane & 15, h = lane >> 4;
+  const bool trail = w >= 1 && w < 8;
+  const int s0 = 2 * (w - 1) + h;          // columns s0, s0 + 14, s0 + 28
+  const bool third = s0 + 28 < kT;
+  auto first_columns = [&](const double (&x)[3]) {      // columns 0-2 for the chain
+    if (s0 < 3) sm.R[s0][r16] = x[0];
+  };
+  int n = 0;
+  for (int I = S.slot_row[slot]; I < S.nt; I = S.next_row[I]) {
+    const int J0 = S.own_first[I];
+    if (tid == kComputeThreads) {
+      if (!wait_geq(S.upd + slot_of(S, I, I - J0), J0 - max(S.ftile[I], S.ftile[J0]), flags))
+        sm.fail = 1;
       __threadfence();
     }
-    __syncthreads();
-    if (sm.fail) return;
-    if (tid < kComputeThreads) panel_task(S, sm, J + 1, J, tid, S.wlstream + (size_t)J * 2 * kTT);
-    else panel_poll(S, sm, J, tid & 31, flags);
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      atomicExch(S.done + slot_of(S, J + 1, 1), 1);
+    bsync();
+    double x[3] = {0.0, 0.0, 0.0};
+    if (trail) {
+      if (!sm.fail) {
+        const double *t = tile_at(S, I, I - J0) + (16 * half + r16) * kT + s0;
+        x[0] = __ldcg(t);
+        x[1] = __ldcg(t + 14);
+        if (third) x[2] = __ldcg(t + 28);
+      }
+      first_columns(x);
+    }
+    bsync();
+    for (int J = J0; J < I; J++, n++) {
+      const int buf = n & 1;
+      if (sm.fail) {       // let the digit warps see it
+        if (w == 0) named_arrive(12 + buf, 32 + kDigitThreads);
+        return;
+      }
+      const bool more = J + 1 < I, upd = more && S.ftile[J + 1] <= J;
+      const int steps = upd ? kT + kLag : kT;
+      double(*W)[17] = sm.W[buf], (*L)[17] = sm.L[buf];
+      if (w >= 8) {
+        const int k = w - 8;
+        const double *st = S.lstream + (size_t)J * kTT + lane;
+        const double *ll = S.wlstream + ((size_t)J * 2 * kTT + kT) + lane;
+        double v = ld_relaxed(st + k * kT), b = 0.0;
+        for (int t = k; t < steps; t += 4) {
+          if (t < kT) {
+            if (lane >= t) {
+              if (unset(v)) v = await_column(st + t * kT, flags);
+              sm.Lc[t & 7][lane] = v;
+            }
+            if (t + 4 < kT && lane >= t + 4) v = ld_relaxed(st + (t + 4) * kT);
+          }
+          if (upd) {
+            const int c = t - kLag;
+            if (c >= 0) {
+              if (unset(b)) b = await_column(ll + c * 2 * kT, flags);
+              sm.Ln[t & 7][lane] = b;
+            }
+            if (c + 4 < kT) b = ld_relaxed(ll + (c + 4) * 2 * kT);
+          }
+          // tile (I, J+1) with the updates of the columns before J
+          if (t == steps - 8 && more && lane == 0 &&
+              !wait_acquire(S.upd + slot_of(S, I, I - J - 1),
+                            max(J - max(S.ftile[I], S.ftile[J + 1]), 0), flags))
+            sm.fail = 1;
+          __syncwarp();
+          named_sync(1 + k, 64);
+        }
+        if (!more && k == 0 && flags[0] != 0 && lane == 0) sm.fail = 1;
+      } else if (w == 0) {
+        double *wl = J + 2 < I || h != 0 ? nullptr
+                                         : (J + 1 == I ? S.wlstream : S.w2stream) +
+                                               (size_t)J * 2 * kTT + 16 * half + r16;
+        if (n >= 2) named_sync(14 + buf, 32 + kDigitThreads);
+        double p1 = 0.0, p2 = 0.0;           // columns t-1, t-2
+        int m3 = 0;                          // t mod 3
+        for (int t = 0; t < steps; t++) {
+          if (t >= 3) named_sync(8 + m3, kComputeThreads);
+          double p = 0.0;
+          if (t < kT) {
+            p = sm.R[t][r16];
+            if (t >= 2) p = fma(-p2, sm.Lc[(t - 2) & 7][t], p);
+            if (t >= 1) p = fma(-p1, sm.Lc[(t - 1) & 7][t], p);
+            W[t][r16] = p;
+            if (wl) publish(wl + t * 2 * kT, p);
+          }
+          named_sync(1 + (t & 3), 64);
+          if (t < kT) {
+            const double inv = sm.Lc[t & 7][t], v = p * inv;
+            L[t][r16] = v;
+            if (lane == 0) sm.inv[buf][t] = inv;
+            if (wl) publish(wl + t * 2 * kT + kT, v);
+          }
+          named_arrive(5 + m3, kComputeThreads);
+          p2 = p1;
+          p1 = p;
+          m3 = m3 == 2 ? 0 : m3 + 1;
+        }
+        named_arrive(12 + buf, 32 + kDigitThreads);
+      } else {
+        double acc[3] = {0.0, 0.0, 0.0}, xn[3] = {0.0, 0.0, 0.0};
+        int m3 = 0;
+        for (int c = 0; c < steps; c++) {
+          named_sync(5 + m3, kComputeThreads);
+          if (c < kT - 3) {
+            const double wc = W[c][r16];
+            const double *lc = sm.Lc[c & 7];
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+              const int s = s0 + 14 * u;
+              if (s >= c + 3 && s < kT) {
+                x[u] = fma(-wc, lc[s], x[u]);
+                if (s == c + 3) sm.R[s][r16] = x[u];
+              }
+            }
+          }
+          if (c < steps - 3) named_arrive(8 + m3, kComputeThreads);
+          if (upd && c >= kLag) {
+            const double pc = W[c - kLag][r16];
+            const double *ln = sm.Ln[c & 7];
+            acc[0] = fma(pc, ln[s0], acc[0]);
+            acc[1] = fma(pc, ln[s0 + 14], acc[1]);
+            if (third) acc[2] = fma(pc, ln[s0 + 28], acc[2]);
+          }
+          if (c == steps - 8 && more) {
+            const double *g = tile_at(S, I, I - J - 1) + (16 * half + r16) * kT + s0;
+            xn[0] = __ldcg(g);
+            xn[1] = __ldcg(g + 14);
+            if (third) xn[2] = __ldcg(g + 28);
+          }
+          m3 = m3 == 2 ? 0 : m3 + 1;
+        }
+#pragma unroll
+        for (int u = 0; u < 3; u++) x[u] = xn[u] - acc[u];
+        first_columns(x);
+      }
+      bsync();
     }
   }
 }
@@ -967,7 +1183,7 @@ __device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, volatile in
     named_sync(7 + s, kFactorThreads);
     const int4 t = sm.task[s];
     if (t.x < 0) return;
-    if (t.x == kPanel) panel_task(S, sm, t.y, t.w, tid, nullptr);
+    if (t.x == kPanel) panel_task(S, sm, t.y, t.w, tid);
     else if (t.x == kPair) pair_task(S, t.w, t.y - t.w, t.z - t.w, tid);
     else if (t.x == kInverse) inverse_task(S, sm, t.w, tid);
     else if (t.x == kCouple) coupling_task(S, sm, t.w, t.z, tid);
@@ -994,16 +1210,23 @@ __device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, volatile in
   }
 }
 
-__global__ void __launch_bounds__(kFactorThreads, 1) k_prof_factor(ProfileSystem S) {
+__global__ void __launch_bounds__(kBlockThreads, 1) k_prof_factor(ProfileSystem S) {
   extern __shared__ __align__(16) unsigned char dyn[];
   FactorSmem &sm = *reinterpret_cast<FactorSmem *>(dyn);
   __shared__ int ticket;
   volatile int *flags = S.flags;
   if (threadIdx.x == 0) ticket = atomicAdd(S.next_task + 1, 1);
   __syncthreads();
-  if (ticket < kDiagBlocks) diag_block(S, sm, ticket, flags);
-  else if (ticket < kDiagBlocks + kPanelBlocks) panel_block(S, sm, ticket - kDiagBlocks, flags);
-  else worker_block(S, sm, flags);
+  const int t = ticket, row = t - kDiagBlocks;
+  if (row >= 0 && row < 2 * S.nslots) {
+    row_block(S, *reinterpret_cast<RowSmem *>(dyn), row >> 1, row & 1, flags);
+    return;
+  }
+  if (t < kDiagBlocks) {
+    if (threadIdx.x < kComputeThreads + kPollThreads) diag_block(S, sm, t, flags);
+  } else if (threadIdx.x < kFactorThreads) {
+    worker_block(S, sm, flags);
+  }
 }
 
 __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem S, int nrhs,
@@ -1161,30 +1384,70 @@ int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &
   return 0;
 }
 
+// Which tile rows the row blocks keep, and from which column: a row from its first
+// column to its last takes a slot of two blocks.  All rows where 28 slots are
+// enough: a row that takes its panels and products from the list needs 14.8 us a
+// column, and the elimination waits for the slowest (one long row behind a
+// constraint held up a 64 x 16 quad block for 150 us).  Beyond that the tile
+// pairs of the list, some 2.7 us each on the blocks that are left, take longer
+// than that a column, and only the two rows next to the diagonal are kept.
+// first[I] >= I: no column; rows of a slot in the order of their first columns.
+constexpr int kMaxSlots = 28;
+void profile_rows(int nt, const std::vector<int> &ftile, std::vector<int> &first,
+                  std::vector<int> &next, std::vector<int> &slot_row) {
+  for (int reach : {nt, 2}) {
+    first.resize(nt);
+    next.assign(nt, nt);
+    slot_row.clear();
+    std::vector<int> order, last;      // last row of each slot
+    for (int I = 0; I < nt; I++) {
+      first[I] = std::max(ftile[I], I - reach);
+      if (first[I] < I) order.push_back(I);
+    }
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int a, int b) { return first[a] < first[b]; });
+    for (int I : order) {
+      size_t k = 0;
+      while (k < last.size() && last[k] > first[I]) k++;
+      if (k == last.size()) {
+        last.push_back(I);
+        slot_row.push_back(I);
+      } else {
+        next[last[k]] = I;
+        last[k] = I;
+      }
+    }
+    if ((int)slot_row.size() <= kMaxSlots) return;
+  }
+}
+
 // The dataflow order of the list's tasks (type, I, K, J): the stream's blocks
-// run the diagonal tiles and the panels (J+1, J).  Column J: the updates of
-// column J-1 that reach column J+1 (the next diagonal tile's last but one
-// first), panel (J+2, J) and its update of tile (J+2, J+1) -- what the stream
-// waits for next --, the other panels, column J's updates of column J+1, the
-// rest of column J-1's trailing update, and the coupling matrices and
-// forward step two columns back.  npairs: tile pairs of each column.
-void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int> &tasks,
-                   std::vector<int> &npairs) {
+// run the diagonal tiles, the row blocks' panels, column J's updates of the next
+// two diagonal tiles and those rows' updates of tile column J+1 by column J.  Column J: the
+// updates of column J-1 that reach column J+1 (the next diagonal tile's last but
+// one first), the other panels, column J's other updates of column J+1, the rest
+// of column J-1's trailing update, and the coupling matrices and forward step two
+// columns back.  npairs: tile pairs of each column in the list.
+void profile_tasks(int nt, int W, const std::vector<int> &ftile, const std::vector<int> &first,
+                   std::vector<int> &tasks, std::vector<int> &npairs) {
   tasks.clear();
   npairs.assign(std::max(nt, 1), 0);
   auto emit = [&](int type, int I, int K, int J) {
     tasks.push_back(type); tasks.push_back(I); tasks.push_back(K); tasks.push_back(J);
     if (type == kPair) npairs[J]++;
   };
-  // the updates of column J whose target column is J+b for b in [blo, bhi]
-  // from row J+alo on (the pair (J+1, J+1) belongs to the stream)
-  auto updates = [&](int J, int blo, int bhi, int alo) {
+  // the updates of column J whose target column is J+b for b in [blo, bhi]; not
+  // the stream's: (J+1, J+1), (J+2, J+2) and the row blocks' of column J+1
+  auto updates = [&](int J, int blo, int bhi) {
     if (J < 0) return;
     const int omax = std::min(W, nt - 1 - J);
     for (int b = blo; b <= std::min(bhi, omax); b++) {
       if (ftile[J + b] > J) continue;
-      for (int a = std::max(b, alo); a <= omax; a++)
-        if (ftile[J + a] <= J) emit(kPair, J + a, J + b, J);
+      for (int a = b; a <= omax; a++) {
+        if (ftile[J + a] > J || (a == b && b <= 2)) continue;
+        if (b == 1 && first[J + a] <= J) continue;
+        emit(kPair, J + a, J + b, J);
+      }
     }
   };
   auto couple = [&](int J) {
@@ -1197,16 +1460,12 @@ void profile_tasks(int nt, int W, const std::vector<int> &ftile, std::vector<int
     emit(kForward, J, J, J);
   };
   for (int J = 0; J < nt; J++) {
-    updates(J - 1, 2, 2, 2);
+    updates(J - 1, 2, 2);
     const int omax = std::min(W, nt - 1 - J);
-    if (omax >= 2 && ftile[J + 2] <= J) {
-      emit(kPanel, J + 2, J + 2, J);
-      if (ftile[J + 1] <= J) emit(kPair, J + 2, J + 1, J);
-    }
-    for (int o = 3; o <= omax; o++)
-      if (ftile[J + o] <= J) emit(kPanel, J + o, J + o, J);
-    updates(J, 1, 1, 3);
-    updates(J - 1, 3, W, 3);
+    for (int o = 1; o <= omax; o++)
+      if (ftile[J + o] <= J && first[J + o] > J) emit(kPanel, J + o, J + o, J);
+    updates(J, 1, 1);
+    updates(J - 1, 3, W);
     couple(J - 2);
   }
   for (int J = std::max(nt - 2, 0); J < nt; J++) couple(J);
@@ -1236,11 +1495,11 @@ int profile_factor(const ProfileSystem &S, cudaStream_t s) {
                                                                nsweep);
   if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
   // all blocks co-resident: the stream waits for list tasks and they for it
-  const int nb = (int)std::min<long>(g_factor_blocks, kDiagBlocks + kPanelBlocks + (long)S.ntasks);
-  if (nb <= kDiagBlocks + kPanelBlocks) return XG_ECUDA;
+  const int nb = (int)std::min<long>(g_factor_blocks, kDiagBlocks + 2 * S.nslots + (long)S.ntasks);
+  if (nb <= kDiagBlocks + 2 * S.nslots) return XG_ECUDA;
   ProfileSystem Sv = S;
   void *args[] = {(void *)&Sv};
-  return cudaLaunchCooperativeKernel((void *)k_prof_factor, dim3(nb), dim3(kFactorThreads), args,
+  return cudaLaunchCooperativeKernel((void *)k_prof_factor, dim3(nb), dim3(kBlockThreads), args,
                                      kFactorSmem, s) == cudaSuccess
              ? 0 : XG_ECUDA;
 }

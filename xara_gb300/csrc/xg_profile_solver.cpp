@@ -49,13 +49,18 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
     return XG_ENOMEM;
   }
   std::vector<int> tasks, npairs;
-  profile_tasks(nt, W, ftile, tasks, npairs);
+  std::vector<int> rows, next, slot_row;   // first columns, then next rows, then the slots
+  profile_rows(nt, ftile, rows, next, slot_row);
+  profile_tasks(nt, W, ftile, rows, tasks, npairs);
+  rows.insert(rows.end(), next.begin(), next.end());
+  rows.insert(rows.end(), slot_row.begin(), slot_row.end());
   const size_t nrow = (size_t)nt * 1024, nslot = (size_t)nt * (W + 1);
   // flags, task counter and tickets, then the per-tile and per-row counters
   const size_t ncount = 8 + 2 * nslot + 4 * (size_t)nt;
   int e = 0;
   e |= ftile_.alloc(ftile.size()) | tasks_.alloc(tasks.size()) | npairs_.alloc(npairs.size());
-  e |= counters_.alloc(ncount) | dig_.alloc(dig) | stream_.alloc(3 * nrow);
+  e |= rows_.alloc(rows.size());
+  e |= counters_.alloc(ncount) | dig_.alloc(dig) | stream_.alloc(5 * nrow);
   e |= L_.alloc(tiles) | Winv_.alloc(nrow) | F_.alloc(nrow) | G_.alloc(nrow);
   e |= E_.alloc(nrow) | H_.alloc(nrow) | Q_.alloc(nrow) | R_.alloc(nrow);
   e |= invD_.alloc((size_t)nt * 32) | piv_.alloc((size_t)nt * 32);
@@ -68,6 +73,8 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
                       cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemcpyAsync(tasks_.p, tasks.data(), tasks.size() * sizeof(int), cudaMemcpyHostToDevice,
                       s) != cudaSuccess ||
+      cudaMemcpyAsync(rows_.p, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, s) !=
+          cudaSuccess ||
       cudaMemcpyAsync(npairs_.p, npairs.data(), npairs.size() * sizeof(int),
                       cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
@@ -88,6 +95,9 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
   S_.cpl = S_.done + nslot; S_.cplq = S_.cpl + nt; S_.colcnt = S_.cplq + nt;
   S_.cplw = S_.colcnt + nt;
   S_.lstream = stream_.p; S_.wlstream = stream_.p + nrow;
+  S_.w2stream = stream_.p + 3 * nrow;
+  S_.own_first = rows_.p; S_.next_row = rows_.p + nt; S_.slot_row = rows_.p + 2 * nt;
+  S_.nslots = (int)slot_row.size();
   S_.counter_bytes = ncount * sizeof(int);
   S_.npairs = npairs_.p; S_.dig = dig_.p;
   S_.min_diag_tol = 1.0e-12;   // ProfileSPDLinDirectSolver.h:49 default
