@@ -38,11 +38,19 @@ struct J2Out {
   int status;
 };
 
+// exp(-delta xi) of the saturating hardening, (sigma0 - sigma_inf) exp(-delta
+// xi): some 25 FP64 operations of the 280 a brick's point takes, where the
+// argument is zero (no plastic strain yet, or delta 0) known to be 1, and without
+// weight where sigma0 equals sigma_inf (any finite value serves).
+__device__ __forceinline__ double j2_decay(const double *p, double xi) {
+  const double t = -p[4] * xi;
+  return t == 0.0 || (p[2] == p[3] && t < 700.0) ? 1.0 : exp(t);
+}
 __device__ __forceinline__ double j2_q(const double *p, double xi) {
-  return p[5] * xi + p[3] + (p[2] - p[3]) * exp(-p[4] * xi);
+  return p[5] * xi + p[3] + (p[2] - p[3]) * j2_decay(p, xi);
 }
 __device__ __forceinline__ double j2_qprime(const double *p, double xi) {
-  return (p[2] - p[3]) * (-p[4]) * exp(-p[4] * xi) + p[5];
+  return (p[2] - p[3]) * (-p[4]) * j2_decay(p, xi) + p[5];
 }
 
 __device__ void j2_return_map(const double *p, const double eps[6], const double epn[6],
@@ -468,6 +476,8 @@ __device__ __constant__ unsigned char kPairB[36] = {
 
 constexpr int kBrickWarps = 1;
 constexpr int kBrickEPW = 4;   // elements per warp
+constexpr int kFFElems = 4, kFFThreads = 36 * kFFElems;   // k_brick_assemble_ff's block
+constexpr int kFFBlocks = 7;                                // and its blocks per SM
 
 // Four elements per warp: Brick::formResidAndTangent (Brick.cpp:844-1021)
 // from the stored point state, formed per node-pair block a <= b and written
@@ -618,7 +628,7 @@ __device__ __forceinline__ double f32_to_f64_scaled(float f, int s) {
   return __hiloint2double((int)(sign | ((unsigned)de << 20) | (m >> 3)), (int)(m << 29));
 }
 
-// The float-float form of k_brick_assemble, four elements per warp.  An
+// The float-float form of k_brick_assemble, four elements per block.  An
 // FP64 FMA holds GB300's FP64 pipe for many cycles; a float-float product
 // (xg_ff.h) costs about twelve single-precision instructions and keeps 46
 // bits of each product, so the tangent carries the reference's values to a
@@ -627,25 +637,32 @@ __device__ __forceinline__ double f32_to_f64_scaled(float f, int s) {
 // scaled by powers of two -- the dN/dx by 2^-eg, the tangent scalings
 // dvol*{a, b/2, c} by 2^-ed, the element's largest magnitudes -- so every
 // product lies near 1 whatever the model's units; the scale comes back
-// exactly in the exponent when a pair is written as a double.
+// exactly in the exponent when an entry is written.
 //
-// Per point first (lane = element, point): the scale exponents, the split
-// tangent scalings and deviatoric direction, dvol * stress.  Then over the
-// eight points (lane = element, node): the node's resisting-force terms in
-// FP64, its split gradient at that point (element-major geo2), the
-// projection h = n . dN/dx and the three scalings, staged in a 3.8 KB
-// slice; then every lane adds the point's terms to the node-pair blocks it
-// owns (144 per warp, 4.5 per lane), whose float-float sums sit in shared
-// memory, transposed so that neighbouring lanes use neighbouring banks.  The
-// task loop is a real loop: with the accumulators in registers its five
-// unrolled copies made a 32 KB loop body that the warps' instruction
-// fetches thrashed.
+// Per point first (thread = element, point): the scale exponents, the split
+// tangent scalings and deviatoric direction, dvol * stress.  Then twice, for
+// four of the eight points at a time: a thread per element, point and node
+// forms the node's resisting-force terms in FP64, its split gradient at that
+// point (element-major geo2), the projection h = n . dN/dx and the three
+// scalings; then a thread per node-pair block (36 of an element) adds the points' terms to its nine sums, which stay in registers, in
+// the points' order.  The matrices leave through shared memory, a float4 a
+// thread in address order.  What bounds it is the issue of the single-precision
+// instructions, some 370 a pair and point (0.6 ms for 196,608 elements at one per
+// cycle and scheduler), and the turns at the FP64 unit between them.  With the sums
+// in shared memory, a warp per four elements and five pairs a lane: 1.58 ms; in
+// registers with eight elements a block, three blocks an SM 1.24, four elements,
+// seven blocks 1.15 ms.
 struct BrickSmemFF {
-  float2 pt[kBrickEPW][8][9];         // per point: dvol*{a, b/2, c}*2^-ed, n[6] (split)
-  double ss[kBrickEPW][8][6];         // per point: dvol * stress
-  float2 nd[5][kBrickEPW][8][3];      // the point being summed: g h u v w per node
-  float2 acc[9][kBrickEPW * 36];      // node-pair block sums (hi, lo), [entry][task]
-  int eg[kBrickEPW], scale[kBrickEPW];
+  union {
+    struct {
+      float2 nd[4][5][kFFElems][8][3];  // per point: g h u v w per node
+      double r[3][kFFElems][4][8];      // and the node's resisting-force terms
+    };
+    float2 K[kFFElems * 576];           // the matrices
+  };
+  float2 pt[kFFElems][8][9];            // per point: dvol*{a, b/2, c}*2^-ed, n[6] (split)
+  double ss[kFFElems][8][6];            // per point: dvol * stress
+  int eg[kFFElems], scale[kFFElems];
 };
 
 // f * 2^s in single precision from the bits: exact where the result is a
@@ -662,17 +679,14 @@ __device__ __forceinline__ float f32_ldexp(float f, int s) {
   return __uint_as_float((u & 0x807fffffu) | ((unsigned)ne << 23));
 }
 
-__global__ void __launch_bounds__(32 * kBrickWarps) k_brick_assemble_ff(ContinuumView v) {
-  __shared__ BrickSmemFF sm_all[kBrickWarps];
-  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  BrickSmemFF &S = sm_all[wi];
-  const int e0 = (blockIdx.x * kBrickWarps + wi) * kBrickEPW;
-  if (e0 >= v.ne) return;
+__global__ void __launch_bounds__(kFFThreads, kFFBlocks) k_brick_assemble_ff(ContinuumView v) {
+  __shared__ __align__(16) BrickSmemFF S;
+  const int tid = threadIdx.x;
+  const int e0 = blockIdx.x * kFFElems, count = min(kFFElems, v.ne - e0);
   const long npts = (long)v.ne * 8;
-  constexpr int kTasks = kBrickEPW * 36;
-  {
-    const int el = lane >> 3, ip = lane & 7, e = e0 + el;
-    const long pt = (long)(e < v.ne ? e : e0) * 8 + ip;
+  if (tid < 8 * kFFElems) {
+    const int el = tid >> 3, ip = tid & 7;
+    const long pt = (long)(e0 + min(el, count - 1)) * 8 + ip;
     int eg = -1000;
 #pragma unroll
     for (int q = 0; q < 24; q++) eg = max(eg, f64_exponent(v.geo[q * npts + pt]));
@@ -700,27 +714,30 @@ __global__ void __launch_bounds__(32 * kBrickWarps) k_brick_assemble_ff(Continuu
     S.pt[el][ip][2] = split2(dc * pd);
 #pragma unroll
     for (int c = 0; c < 6; c++) S.pt[el][ip][3 + c] = split2(v.tan[(3 + c) * npts + pt]);
-    for (int t = lane; t < 9 * kTasks; t += 32) (&S.acc[0][0])[t] = make_float2(0.f, 0.f);
   }
-  __syncwarp();
-  const int el = lane >> 3, a = lane & 7, e = e0 + el;
-  const bool live = e < v.ne;
-  const long ebase = (long)(live ? e : e0) * 8;
-  const float fg = __uint_as_float((unsigned)(127 - S.eg[el]) << 23);
-  double r0 = 0.0, r1 = 0.0, r2 = 0.0;     // resisting force of node a
+  const int te = tid / 36, pp = tid % 36, ta = kPairA[pp], tb = kPairB[pp];
+  float ah[9], al[9], dh = 0.f, dl = 0.f;    // dh: the diagonal's common term
+#pragma unroll
+  for (int q = 0; q < 9; q++) ah[q] = al[q] = 0.f;
+  double r = 0.0;               // threads < 24 kFFElems: component rc of node ra's force
+  const int re = tid / 24, ra = (tid % 24) / 3, rc = tid % 3;
+  __syncthreads();
 #pragma unroll 1
-  for (int ip = 0; ip < 8; ip++) {
-    {
-      // node a of element el at point ip: resisting-force terms (FP64, the
-      // points in order) and the staged float-float terms
+  for (int half = 0; half < 2; half++) {
+    if (tid < 32 * kFFElems) {
+      // node a of element el at point ip: resisting-force terms (FP64) and the
+      // staged float-float terms
+      const int el = tid >> 5, p4 = (tid >> 3) & 3, a = tid & 7, ip = 4 * half + p4;
+      const long pt = (long)(e0 + min(el, count - 1)) * 8 + ip;
+      const float fg = __uint_as_float((unsigned)(127 - S.eg[el]) << 23);
       const double *Sg = S.ss[el][ip];
-      const double g0 = v.geo[a * npts + ebase + ip];
-      const double g1 = v.geo[(8 + a) * npts + ebase + ip];
-      const double g2 = v.geo[(16 + a) * npts + ebase + ip];
-      r0 += g0 * Sg[0] + g1 * Sg[3] + g2 * Sg[5];
-      r1 += g0 * Sg[3] + g1 * Sg[1] + g2 * Sg[4];
-      r2 += g0 * Sg[5] + g1 * Sg[4] + g2 * Sg[2];
-      const float2 *gp = v.geo2 + (ebase + ip) * 24 + a;
+      const double g0 = v.geo[a * npts + pt];
+      const double g1 = v.geo[(8 + a) * npts + pt];
+      const double g2 = v.geo[(16 + a) * npts + pt];
+      S.r[0][el][p4][a] = g0 * Sg[0] + g1 * Sg[3] + g2 * Sg[5];
+      S.r[1][el][p4][a] = g0 * Sg[3] + g1 * Sg[1] + g2 * Sg[4];
+      S.r[2][el][p4][a] = g0 * Sg[5] + g1 * Sg[4] + g2 * Sg[2];
+      const float2 *gp = v.geo2 + pt * 24 + a;
       float2 gi[3];
 #pragma unroll
       for (int i = 0; i < 3; i++) {
@@ -736,77 +753,72 @@ __global__ void __launch_bounds__(32 * kBrickWarps) k_brick_assemble_ff(Continuu
         for (int j = 0; j < 3; j++) ff_madd(P[3 + row[i][j]], gi[j], hh, hl);
         const float hs = __fadd_rn(hh, hl);
         const float2 hi = make_float2(hs, __fsub_rn(hl, __fsub_rn(hs, hh)));
-        S.nd[0][el][a][i] = gi[i];
-        S.nd[1][el][a][i] = hi;
-        S.nd[2][el][a][i] = ff_mul(P[0], gi[i]);
-        S.nd[3][el][a][i] = ff_mul(P[1], gi[i]);
-        S.nd[4][el][a][i] = ff_mul(P[2], hi);
+        S.nd[p4][0][el][a][i] = gi[i];
+        S.nd[p4][1][el][a][i] = hi;
+        S.nd[p4][2][el][a][i] = ff_mul(P[0], gi[i]);
+        S.nd[p4][3][el][a][i] = ff_mul(P[1], gi[i]);
+        S.nd[p4][4][el][a][i] = ff_mul(P[2], hi);
       }
     }
-    __syncwarp();
+    __syncthreads();
+    if (tid < 24 * kFFElems) {
+#pragma unroll
+      for (int p4 = 0; p4 < 4; p4++) r += S.r[rc][re][p4][ra];
+    }
 #pragma unroll 1
-    for (int t = lane; t < kTasks; t += 32) {
-      const int te = t / 36, pp = t % 36;
-      if (e0 + te >= v.ne) continue;
-      const int ta = kPairA[pp], tb = kPairB[pp];
+    for (int p4 = 0; p4 < 4; p4++) {
       float2 gb[3], hb[3], ua[3], va[3], wa[3];
 #pragma unroll
       for (int q = 0; q < 3; q++) {
-        gb[q] = S.nd[0][te][tb][q];
-        hb[q] = S.nd[1][te][tb][q];
-        ua[q] = S.nd[2][te][ta][q];
-        va[q] = S.nd[3][te][ta][q];
-        wa[q] = S.nd[4][te][ta][q];
-      }
-      float ah[9], al[9];
-#pragma unroll
-      for (int q = 0; q < 9; q++) {
-        const float2 c = S.acc[q][t];
-        ah[q] = c.x;
-        al[q] = c.y;
+        gb[q] = S.nd[p4][0][te][tb][q];
+        ua[q] = S.nd[p4][2][te][ta][q];
+        va[q] = S.nd[p4][3][te][ta][q];
+        wa[q] = S.nd[p4][4][te][ta][q];
       }
       // (b/2) dvol dNa . dNb on the diagonal
-      float dh = 0.f, dl = 0.f;
 #pragma unroll
       for (int q = 0; q < 3; q++) ff_madd(va[q], gb[q], dh, dl);
 #pragma unroll
-      for (int i = 0; i < 3; i++) {
+      for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int k = 0; k < 3; k++) {
           ff_madd(ua[i], gb[k], ah[3 * i + k], al[3 * i + k]);
           ff_madd(va[k], gb[i], ah[3 * i + k], al[3 * i + k]);
-          ff_madd(wa[i], hb[k], ah[3 * i + k], al[3 * i + k]);
         }
-        ff_add(dh, dl, ah[4 * i], al[4 * i]);
-      }
+      // c dvol (n . dNa) (n . dNb), zero at an elastic point
+      if (wa[0].x != 0.f || wa[1].x != 0.f || wa[2].x != 0.f) {
 #pragma unroll
-      for (int q = 0; q < 9; q++) S.acc[q][t] = make_float2(ah[q], al[q]);
+        for (int q = 0; q < 3; q++) hb[q] = S.nd[p4][1][te][tb][q];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int k = 0; k < 3; k++) ff_madd(wa[i], hb[k], ah[3 * i + k], al[3 * i + k]);
+      }
     }
-    __syncwarp();   // the slice is restaged for the next point
+    __syncthreads();   // the points' terms are restaged, and then the matrices
   }
-  if (live) {
-    v.Re[(long)e * 24 + 3 * a] = r0;
-    v.Re[(long)e * 24 + 3 * a + 1] = r1;
-    v.Re[(long)e * 24 + 3 * a + 2] = r2;
-  }
-  for (int t = lane; t < kTasks; t += 32) {
-    const int te = t / 36, pp = t % 36;
-    if (e0 + te >= v.ne) continue;
-    const int sc = S.scale[te];
-    const int ta = kPairA[pp], tb = kPairB[pp];
+  if (tid < 24 * count) v.Re[(long)e0 * 24 + tid] = r;
+#pragma unroll
+  for (int i = 0; i < 3; i++) ff_add(dh, dl, ah[4 * i], al[4 * i]);
+  {
     // the element matrix as float pairs in the model's units (the scale put
     // back into the exponents); the gather sums them in float-float
-    float2 *Ke = reinterpret_cast<float2 *>(v.Ke) + (long)(e0 + te) * 576;
+    const int sc = S.scale[te];
+    float2 *Ke = S.K + te * 576;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        const float2 c = S.acc[3 * i + k][t];
-        const float2 kv = make_float2(f32_ldexp(c.x, sc), f32_ldexp(c.y, sc));
+        const float2 kv =
+            make_float2(f32_ldexp(ah[3 * i + k], sc), f32_ldexp(al[3 * i + k], sc));
         Ke[(3 * ta + i) * 24 + 3 * tb + k] = kv;
         if (ta != tb) Ke[(3 * tb + k) * 24 + 3 * ta + i] = kv;
       }
   }
+  __syncthreads();
+  float4 *out = reinterpret_cast<float4 *>(v.Ke) + (long)e0 * 288;
+  const float4 *K4 = reinterpret_cast<const float4 *>(S.K);
+  for (int q = tid; q < 288 * count; q += kFFThreads) out[q] = K4[q];
 }
 
 // Zero-strain trial state (the material constructors call the integrator at
@@ -1156,7 +1168,7 @@ int launch_brick_assemble(const ContinuumView &v, cudaStream_t s) {
   if (v.ne == 0) return 0;
   constexpr int per_block = kBrickWarps * kBrickEPW;
   if (v.geo && v.geo2)
-    k_brick_assemble_ff<<<(v.ne + per_block - 1) / per_block, 32 * kBrickWarps, 0, s>>>(v);
+    k_brick_assemble_ff<<<nblocks(v.ne, kFFElems), kFFThreads, 0, s>>>(v);
   else
     k_brick_assemble<<<(v.ne + per_block - 1) / per_block, 32 * kBrickWarps, 0, s>>>(v);
   return check_launch();
