@@ -32,7 +32,11 @@ namespace xg {
 
 namespace {
 
-constexpr int kAdjWarps = 4;
+// One element (warp) a block: the kernels are bound by the FP64 unit, which serves
+// one warp an operation per 64 cycles and an SM one per 19, so every SM should have
+// its share (420 elements in blocks of four filled 105 of 152 SMs; pass A 427 us,
+// pass B 395, the direct differentiation's 316 and 303, now 389, 361, 296 and 282).
+constexpr int kAdjWarps = 1;
 
 __device__ __forceinline__ double warp_sum_adj(double v) {
 #pragma unroll
