@@ -1414,7 +1414,7 @@ def run_brick(args):
                      "peak_source": peak_kind, "traffic": ncu_traffic("brick", dominant),
                      "algorithmic_bytes_per_launch": alg.get(dominant, alg["phase"]),
                      "limit": "instruction issue on the single-precision pipes, not HBM: the "
-                              "tangent's float-float sums (IPC 2.3 of 4, FMA pipe 42 % under "
+                              "tangent's float-float sums (IPC 2.9 of 4, FMA pipe 53 % under "
                               "ncu: profiles/k_brick_assemble_brick_c2_small.md)"},
         "fp64": {"est_flops_per_step": flops, "achieved_tflops": flops / phase_s / 1e12,
                  "peak_tflops_probe": fp64_peak,

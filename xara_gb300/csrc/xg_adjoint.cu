@@ -32,10 +32,9 @@ namespace xg {
 
 namespace {
 
-// One element (warp) a block: the kernels are bound by the FP64 unit, which serves
-// one warp an operation per 64 cycles and an SM one per 19, so every SM should have
-// its share (420 elements in blocks of four filled 105 of 152 SMs; pass A 427 us,
-// pass B 395, the direct differentiation's 316 and 303, now 389, 361, 296 and 282).
+// One element (warp) a block, so that a slow element holds up no other's place
+// (1,722 elements in blocks of four and of one: pass A 427 and 389 us, pass B 395
+// and 361, the direct differentiation's 316 and 296, 303 and 282).
 constexpr int kAdjWarps = 1;
 
 __device__ __forceinline__ double warp_sum_adj(double v) {

@@ -1200,9 +1200,9 @@ static void fbc_update_as(const FrameView &v, cudaStream_t s) {
 
 // warps: elements (warps) per block, one of 1, 2, 4, 8 (the autotuner's
 // choice; 4 otherwise), fewer in a model of fewer than 1,024 elements a warp: the
-// kernel is bound by the FP64 unit, which serves one warp an operation per 64
-// cycles and an SM one per 19, so a few warps an SM on every SM beat blocks of four
-// on some (420 elements 97 us in blocks of four, 86 in blocks of one)
+// elements take unlike numbers of inner iterations, and a block of four keeps its
+// place until its slowest is done, which only many blocks an SM make up for (1,722
+// elements: 97 us in blocks of four, 86 in blocks of one; 88,377: 1,510 and 1,491)
 int launch_fbc_update(const FrameView &v, cudaStream_t s, int warps) {
   if (v.ne == 0) return 0;
   if (v.nip > kMaxIp) return XG_EINVAL;
