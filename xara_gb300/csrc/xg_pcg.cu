@@ -1268,12 +1268,11 @@ struct NodeKernel {
 };
 template <int KB, int SP, bool kOne>
 NodeKernel node_kernel_ready() {
-  static const bool ready =
-      cudaFuncSetAttribute((const void *)k_pcg_nodes<KB, SP, kOne>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(NodeShared<KB>)) == cudaSuccess;
-  return {ready ? (const void *)k_pcg_nodes<KB, SP, kOne> : nullptr, 32 * NodeShape<KB>::kWarps,
-          (int)sizeof(NodeShared<KB>)};
+  const void *f = (const void *)k_pcg_nodes<KB, SP, kOne>;
+  // the attribute belongs to the current device
+  const bool ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(NodeShared<KB>)) == cudaSuccess;
+  return {ok ? f : nullptr, 32 * NodeShape<KB>::kWarps, (int)sizeof(NodeShared<KB>)};
 }
 // Warps per slice: as many, up to eight, as leave every slice a warp group of
 // its own; vectors in registers as long as that holds.  (More warps on a slice
