@@ -21,6 +21,7 @@
 #include <iterator>
 #include <vector>
 
+#include "xg_block_stream.h"
 #include "xg_ff.h"
 #include "xg_internal.h"
 #include "xg_rcp.h"
@@ -31,13 +32,7 @@ namespace {
 
 constexpr int kPcgThreads = 512;
 constexpr int kPcgMaxBlocks = 160;      // blocks a meeting can hold
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;  // 2 s
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
+constexpr unsigned long long kBarrierTimeoutNs = kCopyTimeoutNs;
 
 // Sense-reversing grid barrier: bar[0] arrivals, bar[1] generation.
 // Returns false (and sets flags[0]) on timeout or when another block did.
@@ -292,23 +287,6 @@ __global__ void __launch_bounds__(kPcgThreads, 2)
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kPcgUnset = 0xFFFFFFFFFFFFFFFFull;   // byte fill 0xFF
 
-// By block order: warps a block, blocks a ring stage, stages a warp, stages
-// whose columns' z is gathered ahead.  A stage
-// is one bulk copy of some 2 KB; the rings take most of an SM's shared memory, some 150 KB in flight.
-template <int KB> struct NodeShape;
-template <> struct NodeShape<1> { static constexpr int kWarps = 16, kGroup = 8, kRing = 4, kAhead = 2; };
-template <> struct NodeShape<2> { static constexpr int kWarps = 16, kGroup = 2, kRing = 5, kAhead = 4; };
-template <> struct NodeShape<3> { static constexpr int kWarps = 16, kGroup = 1, kRing = 5, kAhead = 4; };
-template <> struct NodeShape<6> { static constexpr int kWarps = 4, kGroup = 1, kRing = 5, kAhead = 4; };
-
-// A block of a slice: entry (a, b) of the 32 rows' blocks side by side, and the
-// column nodes.  The node-block copy is an array of these, in the slices' order.
-template <int KB>
-struct BlockRecord {
-  float2 v[KB * KB][32];
-  int col[32];
-};
-
 template <int KB>
 struct NodeShared {
   static constexpr int kWarps = NodeShape<KB>::kWarps, kGroup = NodeShape<KB>::kGroup;
@@ -316,50 +294,13 @@ struct NodeShared {
   BlockRecord<KB> rec[kWarps][kRing][kGroup];
   float2 y[kWarps][KB][32];             // a part's row sums; the parts' residuals as doubles
   double x[kWarps][KB][32];             // the solution (vectors in registers otherwise)
-  unsigned long long full[kWarps][kRing];
+  unsigned long long full[kWarps][kRing + 1];
   double part[2][kWarps];               // the warps' sums
   unsigned top[kWarps];
   double out[4];
   unsigned max;
   int ok[2];                            // by epoch, set by the meeting before
 };
-
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *b) {
-  asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes,
-                                          unsigned long long *b) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(b))
-      : "memory");
-}
-// False when the copy has not come within the limit.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity) {
-  const unsigned a = smem_addr(b);
-  unsigned long long t0 = 0;
-  for (int tries = 0;; tries++) {
-    unsigned done;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if ((tries & 63) == 63) {
-      const unsigned long long now = global_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kBarrierTimeoutNs) return false;
-    }
-  }
-}
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
@@ -598,97 +539,6 @@ __device__ __forceinline__ bool meet(const PcgSystem &S, NodeShared<KB> &E, int 
 // one aligned load.  Each row is summed in float-float (xg_ff.h), a part's
 // groups of blocks alternately into two partial sums, the parts in order: a
 // fixed order.
-
-// A warp's share of the matrix, streamed through its ring: its slices one after
-// another, of each the groups of kGroup blocks part, part + SP, ..., and from
-// the start again for the next SpMV, so that a ring's worth of the next
-// iteration's blocks is there when its z is.  A share no longer than the ring
-// is loaded once.  Lane 0 issues.
-template <int KB, int SP, bool kOne>
-struct BlockStream {
-  static constexpr int kGroup = NodeShape<KB>::kGroup, kRing = NodeShape<KB>::kRing;
-  using Record = BlockRecord<KB>;
-  const PcgSystem &S;
-  Record (*rec)[kGroup];        // the warp's ring
-  unsigned long long *full;
-  int lane, part, first, stride, ns;
-  int total, len;               // groups of the share, stages in use
-  bool ring;                    // more groups than stages
-  int oldest, next;             // stages of the oldest group and the one to wait for next,
-  unsigned phase;               // and the latter's barrier's phase
-  int left, is, wide;           // groups left to issue of the slice in turn, the slice, its
-  const Record *src;            // blocks left, and the next group
-
-  __device__ __forceinline__ int width(int s) const {
-    return (int)((__ldg(S.nb_off + s + 1) - __ldg(S.nb_off + s)) >> 5);
-  }
-  __device__ __forceinline__ int groups(int w) const {
-    const int g = (w + kGroup - 1) / kGroup;
-    return g > part ? (g - part + SP - 1) / SP : 0;
-  }
-  __device__ __forceinline__ void next_slice(int s) {
-    for (is = s;; is += stride) {
-      if (is >= ns) is = first;
-      wide = width(is);
-      left = groups(wide);
-      if (left > 0) break;
-    }
-    wide -= kGroup * part;
-    src = reinterpret_cast<const Record *>(S.nb_vals) + (__ldg(S.nb_off + is) >> 5) + kGroup * part;
-  }
-  __device__ void start() {
-    total = 0;
-    for (int s = first; s < ns; s += stride) total += groups(width(s));
-    len = min(total, kRing);
-    ring = total > kRing;
-    oldest = next = 0;
-    phase = 0u;
-    if (total > 0) {
-      next_slice(first);
-      for (int k = 0; k < len; k++) issue(k);
-    }
-  }
-  __device__ __forceinline__ void issue(int k) {
-    if (lane == 0) {
-      const unsigned bytes =
-          (unsigned)sizeof(Record) * (kGroup == 1 ? 1u : (unsigned)min(kGroup, wide));
-      mbar_expect(full + k, bytes);
-      bulk_load(rec[k], src, bytes, full + k);
-    }
-    src += SP * kGroup;
-    wide -= SP * kGroup;
-    if (--left == 0) {
-      if (kOne) {      // the same slice from its start
-        src -= (long)SP * kGroup * total;
-        wide += SP * kGroup * total;
-        left = total;
-      } else {
-        next_slice(is + stride);
-      }
-    }
-  }
-  // the next group, once it has come
-  __device__ __forceinline__ const Record *get(bool &ok) {
-    ok &= mbar_wait(full + next, phase);
-    const Record *r = rec[next];
-    if (++next == len) {
-      next = 0;
-      phase ^= (unsigned)ring;
-    }
-    return r;
-  }
-  // the warp is done with the oldest group
-  __device__ __forceinline__ void release() {
-    __syncwarp();
-    if (ring) issue(oldest);
-    if (++oldest == len) oldest = 0;
-  }
-  // the copies in flight have come: nothing may land after the block is gone
-  __device__ void drain() {
-    bool ok = true;
-    for (int g = 0; g < len; g++) get(ok);
-  }
-};
 
 // Slice s of 32 node rows belongs to block s % gridDim.x, there to warp group
 // (s / gridDim.x) % (kWarps / SP): SP warps share a slice's blocks in the SpMV,
@@ -963,7 +813,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
         // z of the columns of group g
         auto gather = [&](int g, float2 (&o)[kGroup][KS]) {
           if (g >= groups) return;
-          const BlockRecord<KB> *r = blocks.get(ok);
+          const BlockRecord<KB> *r = blocks.get();
 #pragma unroll
           for (int u = 0; u < kGroup; u++)
             if (kGroup == 1 || kGroup * (part + SP * g) + u < width)
@@ -1052,7 +902,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
           if (L.in) lpq += beta * S.q[L.row] * (S.z[L.row] + beta * S.p[L.row]);
         });
       }
-      if (!ok) {         // a copy that did not come
+      if (blocks.lost()) {         // a copy that did not come
         flags[0] = 2;
         E.ok[epoch & 1] = 0;
       }
