@@ -439,6 +439,8 @@ int xg_measure_fp64_peak(double *tflops);
    values d: y[i] and y_rn[i].  For testing its error bound; no counterpart
    in the reference (ProfileSPDLinDirectSolver divides). */
 int xg_chain_reciprocal_check(int n, const double *d, double *y, double *y_rn);
+/* The same for the tile LDL's pivots (the refinement in integer arithmetic). */
+int xg_pivot_reciprocal_check(int n, const double *d, double *y, double *y_rn);
 
 /* ---- Adjoint of a transient run (no counterpart in the reference; its
         DDM sensitivity, `computeGradients` (runtime/commands/analysis/

@@ -1310,16 +1310,19 @@ extern "C" int xg_measure_fp64_peak(double *tflops) {
 // ---------------------------------------------------------------------------
 namespace xg {
 namespace {
+template <bool kPivot>
 __global__ void k_reciprocal_pair(int n, const double *d, double *y, double *y_rn) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  y[i] = chain_reciprocal(d[i]);
+  if (!kPivot) y[i] = chain_reciprocal(d[i]);
+  else y[i] = reciprocal_out_of_range(d[i]) ? __drcp_rn(d[i]) : wide_reciprocal(d[i]);
   y_rn[i] = __drcp_rn(d[i]);
 }
 }  // namespace
 }  // namespace xg
 
-extern "C" int xg_chain_reciprocal_check(int n, const double *d, double *y, double *y_rn) {
+template <bool kPivot>
+static int reciprocal_check(int n, const double *d, double *y, double *y_rn) {
   if (n < 0 || (n > 0 && (!d || !y || !y_rn))) return XG_EINVAL;
   if (n == 0) return 0;
   double *buf = nullptr;
@@ -1328,7 +1331,7 @@ extern "C" int xg_chain_reciprocal_check(int n, const double *d, double *y, doub
   int rc = 0;
   if (cudaMemcpy(buf, d, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = XG_ECUDA;
   if (!rc) {
-    xg::k_reciprocal_pair<<<(n + 255) / 256, 256>>>(n, buf, buf + n, buf + 2 * (size_t)n);
+    xg::k_reciprocal_pair<kPivot><<<(n + 255) / 256, 256>>>(n, buf, buf + n, buf + 2 * (size_t)n);
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpy(y, buf + n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaMemcpy(y_rn, buf + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -1336,4 +1339,11 @@ extern "C" int xg_chain_reciprocal_check(int n, const double *d, double *y, doub
   }
   cudaFree(buf);
   return rc;
+}
+
+extern "C" int xg_chain_reciprocal_check(int n, const double *d, double *y, double *y_rn) {
+  return reciprocal_check<false>(n, d, y, y_rn);
+}
+extern "C" int xg_pivot_reciprocal_check(int n, const double *d, double *y, double *y_rn) {
+  return reciprocal_check<true>(n, d, y, y_rn);
 }

@@ -20,6 +20,7 @@ namespace xg {
 // the factorisations are the correctly rounded ones; this one only scales
 // the columns during elimination.  xg_chain_reciprocal_check evaluates it
 // beside __drcp_rn for the error-bound test.
+#ifdef __CUDACC__
 __device__ __forceinline__ double chain_reciprocal(double d) {
   const int hi = __double2hiint(d), lo = __double2loint(d);
   const int ahi = hi & 0x7fffffff;
@@ -35,6 +36,7 @@ __device__ __forceinline__ double chain_reciprocal(double d) {
   const double e = fma(-d, x, 1.0);
   return fma(x, fma(e, e, e), x);
 }
+#endif
 
 // 1/d in integer arithmetic, off the FP64 unit, for the tile LDL's chain of
 // pivots: the single-precision hardware reciprocal y0 of d's leading 24 bits
@@ -46,22 +48,23 @@ __device__ __forceinline__ double chain_reciprocal(double d) {
 // chain_reciprocal's three dependent FP64 operations on a unit that takes one
 // per 64 cycles from a warp make 284 cycles; this takes 153.  It holds wherever
 // d and 1/d are normal numbers (reciprocal_out_of_range tells where not); the
-// caller looks where a branch costs it nothing.
+// caller looks where a branch costs it nothing.  The hardware's error of one
+// unit may take the seed of a significand next to 2 below 1/2 (and next to 1
+// to 1): it is held in [1/2, 1], where its 24 bits have one meaning.
+// xg_pivot_reciprocal_check evaluates it on the device.
 __device__ __forceinline__ bool reciprocal_out_of_range(double d) {
   const int be = (__double2hiint(d) >> 20) & 0x7ff;
   return be < 1 || be > 2044;
 }
-__device__ __forceinline__ double wide_reciprocal(double d) {
+// from the bits rb of the seed
+__device__ __forceinline__ double wide_reciprocal_from(double d, unsigned rb) {
   const int hi = __double2hiint(d);
   const unsigned lo = (unsigned)__double2loint(d);
   const int be = (hi >> 20) & 0x7ff;
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;   // m = (mh 2^32 + lo) 2^-52
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r)
-      : "f"(__uint_as_float(0x3f800000u | (((unsigned)hi & 0xfffffu) << 3) | (lo >> 29))));
-  const unsigned rb = __float_as_uint(r);
-  // y0 2^-24, in (1/2, 1]
-  const unsigned y0 = rb >= 0x3f800000u ? 0x1000000u : (rb & 0x7fffffu) | 0x800000u;
+  // y0 2^-24, in [1/2, 1]
+  const unsigned y0 = rb >= 0x3f800000u ? 0x1000000u
+                      : rb < 0x3f000000u ? 0x800000u : (rb & 0x7fffffu) | 0x800000u;
   const unsigned long long p = (unsigned long long)lo * y0;
   const unsigned ph = (unsigned)(p >> 32) + mh * y0;
   const long long e = -(long long)(((unsigned long long)ph << 32) | (unsigned)p);   // e 2^76
@@ -75,4 +78,13 @@ __device__ __forceinline__ double wide_reciprocal(double d) {
       (long long)((((unsigned long long)(2044 - be) << 52) + ((y + 512) >> 10)) |
                   ((unsigned long long)((unsigned)hi & 0x80000000u) << 32)));
 }
+#ifdef __CUDACC__
+__device__ __forceinline__ double wide_reciprocal(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r)
+      : "f"(__uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | (lo >> 29))));
+  return wide_reciprocal_from(d, __float_as_uint(r));
+}
+#endif
 }  // namespace xg
