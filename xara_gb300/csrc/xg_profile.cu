@@ -33,7 +33,8 @@
 // stiffness factor fall off by many orders along a row and FP64 keeps each to
 // its own 53 bits; with seven (63 bits, products cut at 2^-59) the solution
 // of the 10 x 10 x 20 frame lost three digits to the FP64 product, with nine
-// none.  (The idea of error-free digit products: K. Ozaki, T. Ogita, S. Oishi
+// none.  What the fixed point cannot hold are products far below their rows'
+// sizes; those are taken in FP64 (weak_products).  (The idea of error-free digit products: K. Ozaki, T. Ogita, S. Oishi
 // and S. M. Rump, Numer. Algorithms 59, 2012.)
 //
 // Who runs what.  One persistent cooperative launch, a block per SM.  What the
@@ -92,6 +93,8 @@ constexpr int kDiagBlocks = 3;
 constexpr int kPollThreads = 128, kDigitThreads = 128;
 constexpr int kBlockThreads = kComputeThreads + kPollThreads + kDigitThreads;
 constexpr int kBadExp = 1 << 28;       // the exponent of a row with an infinity or a NaN
+constexpr int kZeroExp = -(1 << 27);   // of a row without a digit
+constexpr int kWeakBits = 24;          // below its rows' sizes by these a product is taken in FP64
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -305,7 +308,7 @@ __device__ __forceinline__ void slice_row4(const double (&x)[4], const int (&cs)
   }
   if (q == 0)
     *reinterpret_cast<int *>(dst + kDigitBytes + 4 * r) =
-        bad ? kBadExp : em <= -(1 << 16) ? 0 : em - 1022;
+        bad ? kBadExp : em <= -(1 << 16) ? kZeroExp : em - 1022;
 }
 
 __device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
@@ -346,15 +349,16 @@ __device__ __forceinline__ double fixed_to_double(long long hi, long long lo, in
 // columns n0 + 2 (lane % 4) and the next).  A lane takes columns 8 (lane %
 // 4) .. +7 of its rows as its share of the contraction, the same for both
 // operands, so a digit of a row is one 16-byte load (the operands are
-// written during this launch: read through the L2).
+// written during this launch: read through the L2).  Returns which of the four
+// lie kWeakBits below the product of their rows' sizes (bit k: out[k]).
 __device__ __forceinline__ uint4 frag(const unsigned char *op, int d, int row, int t) {
   return __ldcg(reinterpret_cast<const uint4 *>(op) + (d * kT + row) * 4 + t);
 }
 __device__ __forceinline__ int row_exp(const unsigned char *op, int row) {
   return __ldcg(reinterpret_cast<const int *>(op + kDigitBytes) + row);
 }
-__device__ __forceinline__ void tile_product(const unsigned char *A, const unsigned char *B, int m0,
-                                             int n0, int lane, double (&out)[4]) {
+__device__ __forceinline__ unsigned tile_product(const unsigned char *A, const unsigned char *B,
+                                                 int m0, int n0, int lane, double (&out)[4]) {
   const int g = lane >> 2, t = lane & 3;
   uint4 a0[kDigits], a1[kDigits], b[kDigits];
 #pragma unroll
@@ -379,6 +383,7 @@ __device__ __forceinline__ void tile_product(const unsigned char *A, const unsig
     for (int j = 0; j < kDigits - i; j++)
       mma16816(acc[i + j], a0[i].z, a1[i].z, a0[i].w, a1[i].w, b[j].z, b[j].w);
   }
+  unsigned weak = 0u;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     // weights 2^36 .. 1 of two words; the value is (hi 2^36 + lo) 2^(Ea+Eb-86)
@@ -389,8 +394,14 @@ __device__ __forceinline__ void tile_product(const unsigned char *A, const unsig
       if (u < kDigits - 4) hi += v << (9 * (kDigits - 5 - u));
       else lo += v << (9 * (kDigits - 1 - u));
     }
-    out[k] = fixed_to_double(hi, lo, (k < 2 ? ea0 : ea1) + ((k & 1) ? eb1 : eb0) - 86);
+    const int e = (k < 2 ? ea0 : ea1) + ((k & 1) ? eb1 : eb0);
+    out[k] = fixed_to_double(hi, lo, e - 86);
+    // (a row without digits or with a NaN has no size)
+    if (e > kZeroExp / 2 && e < kBadExp / 2 &&
+        ((__double2hiint(out[k]) >> 20) & 0x7ff) <= max(e + 1023 - kWeakBits, 0))
+      weak |= 1u << k;
   }
+  return weak;
 }
 
 struct FactorSmem {
@@ -579,8 +590,60 @@ __device__ void panel_task(const ProfileSystem &S, FactorSmem &sm, int I, int J,
   panel_store(S, sm.W, sm.L, sm.inv, r, r, q, o, J);
 }
 
+// The entries of out that weak marks, summed again in FP64 from L and the pivots:
+// eight entries at a time, four lanes each with eight columns: 18 operations of 64
+// cycles for a warp where a lane by itself takes 64.  In a 10 x 10 x 20 frame 8 %
+// of the warps have a mark; its load step takes 34.0 ms with them, 33.5 without and
+// 35.2 with the products lane by lane.
+__device__ void weak_products(const ProfileSystem &S, int J, int a, int b, int m0, int n0, int lane,
+                              unsigned weak, double (&out)[4]) {
+  const int group = lane >> 2, t = lane & 3;
+  const double d = __drcp_rn(ld_relaxed(S.lstream + (size_t)J * kTT + lane * (kT + 1)));
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    unsigned marks = __ballot_sync(0xffffffffu, (weak >> u) & 1u);
+    while (marks) {
+      unsigned rest = marks, at = marks;
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        if (k == group) at = rest;
+        rest &= rest - 1;
+      }
+      const bool any = at != 0u;                 // this group's entry: the lane it belongs to
+      const int of = any ? __ffs(at) - 1 : 0;
+      const double2 *x = reinterpret_cast<const double2 *>(
+          tile_at(S, J + a, a) + (m0 + (of >> 2) + 8 * (u >> 1)) * kT + 8 * t);
+      const double2 *y = reinterpret_cast<const double2 *>(
+          tile_at(S, J + b, b) + (n0 + 2 * (of & 3) + (u & 1)) * kT + 8 * t);
+      double2 xv[4], yv[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        xv[k] = __ldcg(x + k);
+        yv[k] = __ldcg(y + k);
+      }
+      double s = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        s = fma(xv[k].x * __shfl_sync(0xffffffffu, d, 8 * t + 2 * k), yv[k].x, s);
+        s = fma(xv[k].y * __shfl_sync(0xffffffffu, d, 8 * t + 2 * k + 1), yv[k].y, s);
+      }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      const int rank = __popc(marks & ((1u << lane) - 1u));
+      const double v = __shfl_sync(0xffffffffu, s, 4 * (rank & 7));
+      if ((marks >> lane & 1u) && rank < 8) out[u] = v;
+      marks = rest;
+    }
+  }
+}
+
 // Phase C on pair (I = J+a, K = J+b), b <= a: A_IK -= P_IJ L_KJ'.  On a
-// diagonal tile the blocks above the diagonal are left out.
+// diagonal tile the blocks above the diagonal are left out.  An entry far below
+// its rows' sizes -- two rows whose large entries do not meet, as of parts that
+// a weak coupling joins -- is where the digits' fixed point holds fewer bits than
+// a double (their error, 2^-77 of the sizes, is a rounding of an entry 2^-24
+// below them, and all of one at 2^-77): it is summed again in FP64 from L and
+// the pivots, so that small entries keep their own 53 bits.
 __device__ void pair_task(const ProfileSystem &S, int J, int a, int b, int tid) {
   const int w = tid >> 5, lane = tid & 31, m0 = (w >> 2) * 16, n0 = (w & 3) * 8;
   if (a == b && n0 >= m0 + 16) return;
@@ -589,7 +652,8 @@ __device__ void pair_task(const ProfileSystem &S, int J, int a, int b, int tid) 
   double2 *c1 = c0 + 4 * kT;
   const double2 v0 = __ldcg(c0), v1 = __ldcg(c1);
   double out[4];
-  tile_product(dig_slot(S, J, a), dig_slot(S, J, b) + kOpBytes, m0, n0, lane, out);
+  const unsigned weak = tile_product(dig_slot(S, J, a), dig_slot(S, J, b) + kOpBytes, m0, n0, lane, out);
+  if (__any_sync(0xffffffffu, weak != 0u)) weak_products(S, J, a, b, m0, n0, lane, weak, out);
   *c0 = make_double2(v0.x - out[0], v0.y - out[1]);
   *c1 = make_double2(v1.x - out[2], v1.y - out[3]);
 }
