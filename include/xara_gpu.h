@@ -394,8 +394,10 @@ int xg_linsoe_get_b(const xg_linsoe *s, double *b);
    in the lower triangle's slot (col, row); get_a returns that lower
    triangle, the upper is zero).  Switching the system zeroes A. */
 int xg_linsoe_set_system(xg_linsoe *s, int system);
-/* BJPCG: PCG to ||r|| <= rtol ||b||; XG_ESOLVE on breakdown or maxit (X
-   holds the last iterate).  PROFILE_SPD: the device LDL' (factored once per
+/* BJPCG: PCG to ||r|| <= rtol ||b||, r by recurrence; the iteration starts
+   again from X while b - A X itself is above 1.05 rtol ||b|| and each start at
+   least halves it.  relres is the recursive one; XG_ESOLVE on breakdown or
+   maxit (X holds the last iterate).  PROFILE_SPD: the device LDL' (factored once per
    matrix: again only after zeroA or addA) and its substitutions; rtol and
    maxit unused, iters = relres = 0; XG_ESOLVE when a pivot fails the
    reference's checks (a first pivot <= 0, a pivot == 0 or |pivot| <=

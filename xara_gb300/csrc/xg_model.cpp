@@ -1669,7 +1669,7 @@ int xg_model::solve(const double *b, double *x, int *iters) {
     if (it > 0) tune_pcg.record(k, ms / it);
     if (tune_pcg.done) pcg_rows = tune_pcg.chosen;
   }
-  prof_end(P_PCG, 1);
+  prof_end(P_PCG, pcg.kb > 0 ? 2 : 1);
   prof_flush();
   last_solver_iters += it;
   if (iters) *iters = it;
