@@ -73,3 +73,32 @@ def test_the_iteration_limit_holds():
         assert s.solve(rtol=RTOL, maxit=full - 20)[1] == full - 20
         with pytest.raises(gpu.XaraGpuError):
             s.solve(rtol=RTOL, maxit=1000)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kb", [1, 3])
+@pytest.mark.parametrize("size", [1e-148, 1e-140, 1e140, 1e150])
+def test_loads_at_the_ends_of_the_range(kb, size):
+    """r.z and p.q of such loads have no normal reciprocal (they are subnormal at
+    the end of the smallest ones' solve, above 2^1022 at the start of the
+    largest's), but their quotients are ordinary numbers.  The squares of the smallest
+    residuals resolve r to 2^-537, 1e-14 of b."""
+    sp = pytest.importorskip("scipy.sparse")
+    n, ids, c = _grid(12, kb, 1.0, 1.0, 3)
+    a = [([[w, -w], [-w, w]], p) for p, w in zip(ids, c)] + [([[0.3]], [k]) for k in range(n)]
+    A = np.zeros((n, n))
+    for m, p in a:
+        for i, r in enumerate(p):
+            for j, q in enumerate(p):
+                if r >= 0 and q >= 0:
+                    A[r, q] += m[i][j]
+    P = sp.csr_matrix(A != 0)
+    P.sort_indices()
+    b = np.random.default_rng(2).normal(size=n)
+    with gpu.LinearSystem(P.indptr.astype(np.int32), P.indices.astype(np.int32),
+                          np.arange(0, n + 1, kb)) as s:
+        for m, p in a:
+            s.add_a(m, p)
+        s.set_b(b * size)
+        x = s.solve(rtol=RTOL, maxit=2000)[0] / size
+    assert np.linalg.norm(b - A @ x) <= 2 * RTOL * np.linalg.norm(b)

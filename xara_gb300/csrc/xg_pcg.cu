@@ -298,7 +298,7 @@ struct NodeShared {
   unsigned long long full[kWarps][kRing + 1];
   double part[2][kWarps];               // the warps' sums
   unsigned top[kWarps];
-  double out[4];
+  double out[5];
   unsigned max;
   int ok[2];                            // by epoch, set by the meeting before
 };
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
       // alpha = rz / p.q
       ok = meet<1>(S, E, epoch, lpq, 0.0, 0u, flags, [&](int, double t) {
              E.out[0] = t;
-             E.out[1] = rz * chain_reciprocal(t);
+             E.out[1] = reciprocal_out_of_range(t) ? rz / t : rz * chain_reciprocal(t);
            }, chunked, longs);
       if (!ok) break;
       if (!(E.out[0] > 0.0)) { status = -1; break; }
@@ -993,13 +993,14 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
       const double rz_inv = E.out[2];
       ok = meet<2>(S, E, epoch, lrz, lrr, mz, flags, [&](int q, double t) {
         E.out[q] = t;
+        if (q == 0 && reciprocal_out_of_range(rz)) E.out[4] = t / rz;
         if (q == 1) E.out[3] = converged(t) ? 1.0 : 0.0;
       });
       if (!ok) break;
       rr = E.out[1];
       it++;
       if (E.out[3] != 0.0) { status = 1; break; }
-      beta = E.out[0] * rz_inv;
+      beta = reciprocal_out_of_range(rz) ? E.out[4] : E.out[0] * rz_inv;
       rz = E.out[0];
       all64 |= !isfinite(mag_bound(E.max));
       next = split_exponent(mag_bound(E.max));
