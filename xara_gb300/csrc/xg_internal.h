@@ -194,6 +194,7 @@ struct ProfileSystem {
   // none), [nslots] a slot's first row
   const int *own_first, *next_row, *slot_row;
   int nslots;
+  int sms;                 // of the device the system lies on
   // right-hand sides whose forward sweep runs inside the factorisation
   // (fwd_nrhs 0: none)
   int fwd_nrhs;
@@ -209,6 +210,9 @@ void profile_tasks(int nt, int W, const std::vector<int> &ftile, const std::vect
 size_t profile_tile_doubles(int nt, int W);
 size_t profile_digit_bytes(int W);
 int profile_tile_edge();
+// The current device made ready for a factorisation (its kernel's shared memory is
+// an attribute of the device's context), and its SM count.
+int profile_device(int *sms);
 // Factor the CSR values into the tiles, with the forward sweep of
 // fwd_nrhs right-hand sides b.  Enqueued only; profile_status tells the
 // outcome.

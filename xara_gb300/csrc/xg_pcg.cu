@@ -1144,24 +1144,20 @@ __global__ void k_pack_blocks(PcgSystem S) {
   S.blk_ff[i] = ok ? 1 : 0;
 }
 
-// co-resident blocks of the CSR solve; blocks of the node solve (one per SM)
-int g_csr_blocks = -1, g_node_blocks = -1;
-
+// co-resident blocks of the CSR solve; blocks of the node solve (one per SM): of
+// the current device
+int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
 int csr_blocks() {
-  if (g_csr_blocks < 0) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg, kPcgThreads, 0);
-    g_node_blocks = std::min(sms, kPcgMaxBlocks);
-    g_csr_blocks = sms * std::max(per, 1);
-  }
-  return g_csr_blocks;
+  int per = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg, kPcgThreads, 0);
+  return sm_count() * std::max(per, 1);
 }
-int node_blocks() {
-  csr_blocks();
-  return g_node_blocks;
-}
+int node_blocks() { return std::min(sm_count(), kPcgMaxBlocks); }
 
 struct NodeKernel {
   const void *f;

@@ -1435,8 +1435,6 @@ __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem 
   }
 }
 
-int g_factor_blocks = -1;
-
 }  // namespace
 
 int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &ftile, int &nt,
@@ -1547,27 +1545,27 @@ size_t profile_tile_doubles(int nt, int W) { return (size_t)nt * (W + 1) * kTT; 
 size_t profile_digit_bytes(int W) { return (size_t)kRing * W * kSlotBytes; }
 int profile_tile_edge() { return kT; }
 
+int profile_device(int *sms) {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess &&
+                 cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_prof_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kFactorSmem) == cudaSuccess
+             ? 0 : XG_ECUDA;
+}
+
 int profile_factor(const ProfileSystem &S, cudaStream_t s) {
   if (S.n == 0) return 0;
-  if (g_factor_blocks < 0) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(k_prof_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kFactorSmem) != cudaSuccess)
-      return XG_ECUDA;
-    g_factor_blocks = sms;
-  }
   if (S.fwd_nrhs < 0 || S.fwd_nrhs > 4) return XG_EINVAL;
   // the sweeps' values: forward ones published inside the factorisation,
   // backward ones by the solve behind it
   const size_t nsweep = 4 * (size_t)S.fwd_nrhs * S.nt * kT;
-  const long nprep = std::min<long>(8 * (long)g_factor_blocks, (long)S.nt * kT / 8);
+  const long nprep = std::min<long>(8 * (long)S.sms, (long)S.nt * kT / 8);
   k_prof_prepare<<<(int)std::max<long>(nprep, 1), 256, 0, s>>>(S, S.counter_bytes / sizeof(int),
                                                                nsweep);
   if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
   // all blocks co-resident: the stream waits for list tasks and they for it
-  const int nb = (int)std::min<long>(g_factor_blocks, kDiagBlocks + 2 * S.nslots + (long)S.ntasks);
+  const int nb = (int)std::min<long>(S.sms, kDiagBlocks + 2 * S.nslots + (long)S.ntasks);
   if (nb <= kDiagBlocks + 2 * S.nslots) return XG_ECUDA;
   ProfileSystem Sv = S;
   void *args[] = {(void *)&Sv};

@@ -39,6 +39,11 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
     record_error("ProfileSPD: cudaMemGetInfo failed");
     return XG_ECUDA;
   }
+  int sms = 0;
+  if (profile_device(&sms) != 0) {
+    record_error("ProfileSPD: the device refuses the factorisation's shared memory");
+    return XG_ECUDA;
+  }
   const size_t dig = profile_digit_bytes(W);
   if ((tiles + (size_t)nt * 32 * 6) * sizeof(double) > free_b / 2) {
     char msg[160];
@@ -98,6 +103,7 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
   S_.w2stream = stream_.p + 3 * nrow;
   S_.own_first = rows_.p; S_.next_row = rows_.p + nt; S_.slot_row = rows_.p + 2 * nt;
   S_.nslots = (int)slot_row.size();
+  S_.sms = sms;
   S_.counter_bytes = ncount * sizeof(int);
   S_.npairs = npairs_.p; S_.dig = dig_.p;
   S_.min_diag_tol = 1.0e-12;   // ProfileSPDLinDirectSolver.h:49 default
