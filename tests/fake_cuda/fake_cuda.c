@@ -1,8 +1,9 @@
 /* A stand-in for the CUDA runtime calls that a linear system makes, preloaded
    by tests/test_fake_device.py: device memory is host memory, nothing is run.
-   A cooperative launch is refused as a device refuses it: more blocks than SMs
-   (one a SM), more shared memory than was asked for on the device at hand, or
-   the FAKE_REFUSE'th one (0: none) whatever it is. */
+   A cooperative launch is refused as a device refuses it: more blocks than fit
+   (one a SM of more than half its shared memory, else four), more shared memory
+   than was asked for on the device at hand, or the FAKE_REFUSE'th one (0: none)
+   whatever it is. */
 #include <stdlib.h>
 #include <string.h>
 
@@ -47,5 +48,5 @@ int cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3 b, void **a, size_t 
   for (k = 0; k < nattr; k++)
     if (attr[k].f == f && attr[k].dev == device && (size_t)attr[k].bytes >= n) ok = 1;
   if (++launches == env("FAKE_REFUSE", 0)) return 999;
-  return !ok ? 1 : (int)g.x > env("FAKE_SMS", 152) ? 720 : 0;
+  return !ok ? 1 : (int)g.x > env("FAKE_SMS", 152) * (n > 114 * 1024 ? 1 : 4) ? 720 : 0;
 }

@@ -60,3 +60,20 @@ def test_each_device_gets_its_attributes(run):
             rt.cudaSetDevice(dev)
             assert code(300, 40, LDL) == (0, ""), code(300, 40, LDL)
     """)
+
+
+@pytest.mark.parametrize("sms", [8, 9, 12, 20, 59, 60, 132])
+def test_small_devices_factor_too(run, sms):
+    """One block a SM and one at least for the list, whatever the envelope: one
+    tile, one neighbour, 25 and 29 tile rows below the diagonal, a long row's."""
+    run(f"""
+        for n, band in ((20, 5), (300, 20), (1000, 24 * 32), (1000, 29 * 32), (1000, 999)):
+            assert code(n, band, LDL) == (0, ""), (n, band, code(n, band, LDL))
+    """, FAKE_SMS=sms)
+
+
+def test_too_small_a_device_is_named(run):
+    run("""
+        c, text = code(300, 100, LDL)
+        assert c < 0 and "needs 8 SMs" in text and "has 7" in text, (c, text)
+    """, FAKE_SMS=7)

@@ -203,8 +203,9 @@ struct ProfileSystem {
 };
 int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &ftile, int &nt,
                  int &W);
-void profile_rows(int nt, const std::vector<int> &ftile, std::vector<int> &first,
-                  std::vector<int> &next, std::vector<int> &slot_row);
+// Returns the blocks a factorisation runs on at least.
+int profile_rows(int nt, const std::vector<int> &ftile, int sms, std::vector<int> &first,
+                 std::vector<int> &next, std::vector<int> &slot_row);
 void profile_tasks(int nt, int W, const std::vector<int> &ftile, const std::vector<int> &first,
                    std::vector<int> &tasks, std::vector<int> &npairs);
 size_t profile_tile_doubles(int nt, int W);

@@ -1462,9 +1462,12 @@ int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &
 // pairs of the list, some 2.7 us each on the blocks that are left, take longer
 // than that a column, and only the two rows next to the diagonal are kept.
 // first[I] >= I: no column; rows of a slot in the order of their first columns.
+// A device of fewer SMs than 152 gets its share of the slots, so that blocks for the
+// list are left; two rows next to the diagonal take two slots whatever the system.
 constexpr int kMaxSlots = 28;
-void profile_rows(int nt, const std::vector<int> &ftile, std::vector<int> &first,
-                  std::vector<int> &next, std::vector<int> &slot_row) {
+int profile_rows(int nt, const std::vector<int> &ftile, int sms, std::vector<int> &first,
+                 std::vector<int> &next, std::vector<int> &slot_row) {
+  const int most = std::min(kMaxSlots, (sms - kDiagBlocks) * kMaxSlots / (152 - kDiagBlocks));
   for (int reach : {nt, 2}) {
     first.resize(nt);
     next.assign(nt, nt);
@@ -1487,8 +1490,9 @@ void profile_rows(int nt, const std::vector<int> &ftile, std::vector<int> &first
         last[k] = I;
       }
     }
-    if ((int)slot_row.size() <= kMaxSlots) return;
+    if ((int)slot_row.size() <= most) break;
   }
+  return kDiagBlocks + 2 * (int)slot_row.size() + 1;
 }
 
 // The dataflow order of the list's tasks (type, I, K, J): the stream's blocks
@@ -1566,7 +1570,6 @@ int profile_factor(const ProfileSystem &S, cudaStream_t s) {
   if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
   // all blocks co-resident: the stream waits for list tasks and they for it
   const int nb = (int)std::min<long>(S.sms, kDiagBlocks + 2 * S.nslots + (long)S.ntasks);
-  if (nb <= kDiagBlocks + 2 * S.nslots) return XG_ECUDA;
   ProfileSystem Sv = S;
   void *args[] = {(void *)&Sv};
   return cudaLaunchCooperativeKernel((void *)k_prof_factor, dim3(nb), dim3(kBlockThreads), args,

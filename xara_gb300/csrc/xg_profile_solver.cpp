@@ -55,7 +55,14 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
   }
   std::vector<int> tasks, npairs;
   std::vector<int> rows, next, slot_row;   // first columns, then next rows, then the slots
-  profile_rows(nt, ftile, rows, next, slot_row);
+  const int blocks = profile_rows(nt, ftile, sms, rows, next, slot_row);
+  if (blocks > sms) {
+    char msg[160];
+    snprintf(msg, sizeof msg, "ProfileSPD: the factorisation needs %d SMs, the device has %d",
+             blocks, sms);
+    record_error(msg);
+    return XG_ECUDA;
+  }
   profile_tasks(nt, W, ftile, rows, tasks, npairs);
   rows.insert(rows.end(), next.begin(), next.end());
   rows.insert(rows.end(), slot_row.begin(), slot_row.end());
