@@ -77,3 +77,13 @@ def test_too_small_a_device_is_named(run):
         c, text = code(300, 100, LDL)
         assert c < 0 and "needs 8 SMs" in text and "has 7" in text, (c, text)
     """, FAKE_SMS=7)
+
+
+@pytest.mark.parametrize("system,launch", [("LDL", 1), ("LDL", 2), ("PCG", 1)])
+def test_a_refused_launch_is_no_failed_solve(run, system, launch):
+    """XG_ECUDA (-2) with its own text, not XG_ESOLVE (-4) or a wait that timed out."""
+    run(f"""
+        c, text = code(300, 40, {system})
+        assert c == -2 and "timed out" not in text and "pivot" not in text, (c, text)
+        assert "CUDA" in text, text
+    """, FAKE_REFUSE=launch)

@@ -338,8 +338,9 @@ static int linsoe_solve_profile(xg_linsoe *s, int *iters, double *relres) {
         snprintf(msg, sizeof msg, "xg_linsoe_solve: ProfileSPD pivot %d fails the check (aii == "
                  "0, |aii| <= 1e-12, or a first pivot <= 0)", bad);
       else
-        snprintf(msg, sizeof msg, "xg_linsoe_solve: ProfileSPD factorisation wait timed out");
-      return lfail(XG_ESOLVE, msg);
+        snprintf(msg, sizeof msg, "xg_linsoe_solve: ProfileSPD factorisation %s",
+                 e == XG_ESOLVE ? "wait timed out" : "did not run: a CUDA call failed");
+      return lfail(e, msg);
     }
     s->prof_factored = true;
   } else if (int e = s->prof.solve(1, &bp, &xp, st)) {
@@ -380,6 +381,8 @@ int xg_linsoe_solve(xg_linsoe *s, double rtol, int maxit, int *iters, double *re
     return lfail(XG_ECUDA, "xg_linsoe_solve: copy of X failed");
   if (iters) *iters = it;
   if (relres) *relres = rr;
+  if (r && r != XG_ESOLVE)
+    return lfail(r, "xg_linsoe_solve: PCG did not run: a CUDA call failed");
   if (r) {
     char msg[128];
     snprintf(msg, sizeof msg, "xg_linsoe_solve: PCG did not converge (%d iterations, %.3e)", it,

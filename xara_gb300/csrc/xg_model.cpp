@@ -1526,24 +1526,27 @@ int xg_model::solve_profile(int nrhs, const double *const *b, double *const *x) 
     // the tangent is new and its right-hand sides are known: the forward
     // sweep runs inside the factorisation, then the backward sweep
     prof_begin(P_LDL_FACTOR);
-    RET(envelope.factor_forward(nrhs, b, stream));
+    int bad = -1, r = envelope.factor_forward(nrhs, b, stream);
     prof_end(P_LDL_FACTOR, 2);
     prof_begin(P_LDL_SOLVE);
-    int bad = -1;
-    const int r = envelope.solve_backward(nrhs, x, stream, &bad);
+    if (!r) r = envelope.solve_backward(nrhs, x, stream, &bad);
     prof_end(P_LDL_SOLVE, 1);
     if (r) {
       if (bad >= 0) return fail(XG_ESOLVE, "ProfileSPD: pivot %d fails the check (aii == 0, "
                                 "|aii| <= 1e-12, or a first pivot <= 0)", bad);
-      return fail(r, "ProfileSPD: factorisation barrier timed out");
+      return fail(r, r == XG_ESOLVE ? "ProfileSPD: factorisation wait timed out"
+                                    : "ProfileSPD: factorisation did not run: a CUDA call failed");
     }
     prof_factored = true;
     prof_flush();
     return 0;
   }
   prof_begin(P_LDL_SOLVE);
-  RET(envelope.solve(nrhs, b, x, stream));
+  const int r = envelope.solve(nrhs, b, x, stream);
   prof_end(P_LDL_SOLVE, 1);
+  if (r)
+    return fail(r, r == XG_ESOLVE ? "ProfileSPD: substitution wait timed out"
+                                  : "ProfileSPD: substitution did not run: a CUDA call failed");
   prof_flush();
   return 0;
 }
@@ -1673,6 +1676,7 @@ int xg_model::solve(const double *b, double *x, int *iters) {
   prof_flush();
   last_solver_iters += it;
   if (iters) *iters = it;
+  if (r != 0 && r != XG_ESOLVE) return fail(r, "PCG did not run: a CUDA call failed");
   if (r != 0)
     return fail(XG_ESOLVE, "PCG did not converge: %d iterations, relative residual %.3e", it,
                 relres);
