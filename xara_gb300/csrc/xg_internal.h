@@ -177,6 +177,7 @@ struct ProfileSystem {
   double *sweep;           // [4*4*nt*32] values published by the sweeps (y, c, x, c')
   int *flags;              // [4]; the counters above follow it in one block
   size_t counter_bytes;    // of that block
+  unsigned long long wait_ns;  // how long a wait for another block may last
   double min_diag_tol;
   // per tile row J, for the substitutions (row-major 32 x 32 each,
   // [nt*1024]): W_J = L_JJ^-T, F_J = L_JJ^-1 L_J,J-1, G_J = L_JJ^-T

@@ -78,7 +78,6 @@ constexpr int kT = 32;                 // tile edge
 constexpr int kTT = kT * kT;
 constexpr int kComputeThreads = 256;   // the eight computing warps of a block
 constexpr int kFactorThreads = kComputeThreads + 32;
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;  // 2 s
 
 // digits of a tile operand: [kDigits][row][column] halves, then the rows'
 // exponents
@@ -147,27 +146,34 @@ __device__ __forceinline__ void named_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
+// The status words, and how long a wait may last.
+struct Waits {
+  volatile int *p;
+  unsigned long long ns;
+  __device__ __forceinline__ volatile int &operator[](int k) const { return p[k]; }
+};
+
 // Wait until *p >= target (one thread); false on a raised error flag or after
-// kBarrierTimeoutNs (flags[0] = 2).
-__device__ __noinline__ bool wait_slow(const int *p, int target, volatile int *flags) {
+// the limit (flags[0] = 2).
+__device__ __noinline__ bool wait_slow(const int *p, int target, Waits flags) {
   const volatile int *vp = p;
   const unsigned long long t0 = global_ns();
   for (;;) {
     for (int k = 0; k < 32; k++)
       if (*vp >= target) return true;
     if (flags[0] != 0) return false;
-    if (global_ns() - t0 > kBarrierTimeoutNs) {
+    if (global_ns() - t0 > flags.ns) {
       flags[0] = 2;
       return false;
     }
   }
 }
-__device__ __forceinline__ bool wait_geq(const int *p, int target, volatile int *flags) {
+__device__ __forceinline__ bool wait_geq(const int *p, int target, Waits flags) {
   return *(const volatile int *)p >= target || wait_slow(p, target, flags);
 }
 
 // The same with the order of the loads behind it (half the time of a fence).
-__device__ __forceinline__ bool wait_acquire(const int *p, int target, volatile int *flags) {
+__device__ __forceinline__ bool wait_acquire(const int *p, int target, Waits flags) {
   for (int k = 0;; k++) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -197,19 +203,19 @@ __device__ __forceinline__ bool unset(double v) {
 // the clock between two loads keeps them from crowding the L2 (981 against
 // 1,108 us a backward sweep of 454 tile rows); await_column for the few warps
 // that follow the factorisation's stream.
-__device__ __forceinline__ double await_slow(const double *p, volatile int *flags) {
+__device__ __forceinline__ double await_slow(const double *p, Waits flags) {
   const unsigned long long t0 = global_ns();
   for (;;) {
     const double v = ld_relaxed(p);
     if (!unset(v)) return v;
     if (flags[0] != 0) return 0.0;
-    if (global_ns() - t0 > kBarrierTimeoutNs) {
+    if (global_ns() - t0 > flags.ns) {
       flags[0] = 2;
       return 0.0;
     }
   }
 }
-__device__ __forceinline__ double await_column(const double *p, volatile int *flags) {
+__device__ __forceinline__ double await_column(const double *p, Waits flags) {
   const unsigned long long t0 = global_ns();
   for (;;) {
 #pragma unroll 1
@@ -218,7 +224,7 @@ __device__ __forceinline__ double await_column(const double *p, volatile int *fl
       if (!unset(v)) return v;
     }
     if (flags[0] != 0) return 0.0;
-    if (global_ns() - t0 > kBarrierTimeoutNs) {
+    if (global_ns() - t0 > flags.ns) {
       flags[0] = 2;
       return 0.0;
     }
@@ -226,7 +232,7 @@ __device__ __forceinline__ double await_column(const double *p, volatile int *fl
 }
 
 // p[0], p[8], p[16], p[24] (the four loads in flight together)
-__device__ __forceinline__ void await4(const double *p, double v[4], volatile int *flags) {
+__device__ __forceinline__ void await4(const double *p, double v[4], Waits flags) {
 #pragma unroll
   for (int m = 0; m < 4; m++) v[m] = ld_relaxed(p + 8 * m);
 #pragma unroll
@@ -540,7 +546,7 @@ __device__ __forceinline__ void panel_store(const ProfileSystem &S, const double
 // ahead of the others; one barrier a column.  Afterwards L goes
 // to the tile and both, as digits, to the ring slot.
 __device__ void panel_poll(const ProfileSystem &S, FactorSmem &sm, int J, int lane,
-                           volatile int *flags) {
+                           Waits flags) {
   const double *st = S.lstream + (size_t)J * kTT;
   double v = ld_relaxed(st + lane);
   for (int c = 0; c < kT; c++) {
@@ -766,11 +772,11 @@ __device__ __forceinline__ int done_count(const ProfileSystem &S, int I, int J) 
   return I > J && J >= S.own_first[I] ? 2 * kDigitThreads / 32 : 1;
 }
 __device__ __forceinline__ bool wait_done(const ProfileSystem &S, int I, int J,
-                                          volatile int *flags) {
+                                          Waits flags) {
   return wait_geq(S.done + slot_of(S, I, I - J), done_count(S, I, J), flags);
 }
 enum { kPanel = 1, kPair = 2, kInverse = 5, kCouple = 6, kForward = 7, kCouple2 = 8 };
-__device__ bool wait_task(const ProfileSystem &S, int4 t, volatile int *flags) {
+__device__ bool wait_task(const ProfileSystem &S, int4 t, Waits flags) {
   const int type = t.x, I = t.y, K = t.z, J = t.w;
   if (type == kPanel)     // the columns of L_JJ are polled inside the task
     return (J < kRing || wait_geq(S.colcnt + J - kRing, S.npairs[J - kRing], flags)) &&
@@ -831,7 +837,7 @@ __device__ __forceinline__ double rhs_at(const ProfileSystem &S, int q, int i) {
 // y_J-2, published to the sweep's scratch (y, c) for the rows after it and
 // for the backward sweep.
 __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
-                            volatile int *flags) {
+                            Waits flags) {
   const int tid = threadIdx.x;
   const int r = tid >> 3, g = tid & 7;
   const int nrhs = S.fwd_nrhs, ls = S.nt * kT;
@@ -903,7 +909,7 @@ __device__ bool forward_row(const ProfileSystem &S, int J, double (*rb)[kT],
 // eight warps); four warps poll, a column in four each, since a look at a published
 // value takes longer than a column.
 constexpr int kSlots = 17;
-__device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, volatile int *flags) {
+__device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, Waits flags) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid >> 3, q = tid & 7;
   const TrailEntries te = trail_entries(warp, lane);
@@ -989,7 +995,7 @@ __device__ void diag_block(const ProfileSystem &S, FactorSmem &sm, int first, vo
                                               : (d == 0.0 || fabs(d) <= S.min_diag_tol));
       const unsigned which = __ballot_sync(0xffffffffu, bad);
       if (which && tid == 0) {
-        if (atomicCAS((int *)flags, 0, 4) == 0) {
+        if (atomicCAS((int *)flags.p, 0, 4) == 0) {
           flags[1] = J * kT + __ffs(which) - 1;
           __threadfence();
           flags[0] = 3;
@@ -1042,7 +1048,7 @@ struct RowSmem {
 };
 static_assert(sizeof(RowSmem) <= kFactorSmem, "");
 __device__ void row_digits(const ProfileSystem &S, RowSmem &sm, int slot, int half,
-                           volatile int *flags) {
+                           Waits flags) {
   const int tid = threadIdx.x - kComputeThreads - kPollThreads, lane = tid & 31;
   int n = 0;
   for (int I = S.slot_row[slot]; I < S.nt; I = S.next_row[I])
@@ -1068,7 +1074,7 @@ __device__ void row_digits(const ProfileSystem &S, RowSmem &sm, int slot, int ha
 }
 
 __device__ void row_block(const ProfileSystem &S, RowSmem &sm, int slot, int half,
-                          volatile int *flags) {
+                          Waits flags) {
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   if (tid == 0) sm.fail = 0;
   __syncthreads();
@@ -1083,10 +1089,14 @@ __device__ void row_block(const ProfileSystem &S, RowSmem &sm, int slot, int hal
   auto first_columns = [&](const double (&x)[3]) {      // columns 0-2 for the chain
     if (s0 < 3) sm.R[s0][r16] = x[0];
   };
-  int n = 0;
+  int n = 0, front = 0;
   for (int I = S.slot_row[slot]; I < S.nt; I = S.next_row[I]) {
     const int J0 = S.own_first[I];
     if (tid == kComputeThreads) {
+      // the eliminations up to the row's first column but one, one after another: the
+      // slot may be idle for as long as those take, its wait's limit is for each
+      while (front < J0 - 1 && wait_done(S, front, front, flags)) front++;
+      front = I - 1;      // when this row's last panel is solved
       if (!wait_geq(S.upd + slot_of(S, I, I - J0), J0 - max(S.ftile[I], S.ftile[J0]), flags))
         sm.fail = 1;
       __threadfence();
@@ -1218,7 +1228,7 @@ __device__ void row_block(const ProfileSystem &S, RowSmem &sm, int slot, int hal
 // waits for its operands while warps 0-7 run the present one (barriers 7-8:
 // a task is ready, 5-6: its slot is free again); during a panel, which lasts
 // as long as its column's elimination, it polls the column instead.
-__device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, volatile int *flags) {
+__device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, Waits flags) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 8) {
     int pending = 0;
@@ -1286,7 +1296,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_prof_factor(ProfileSystem 
   extern __shared__ __align__(16) unsigned char dyn[];
   FactorSmem &sm = *reinterpret_cast<FactorSmem *>(dyn);
   __shared__ int ticket;
-  volatile int *flags = S.flags;
+  const Waits flags{S.flags, S.wait_ns};
   if (threadIdx.x == 0) ticket = atomicAdd(S.next_task + 1, 1);
   __syncthreads();
   const int t = ticket, row = t - kDiagBlocks;
@@ -1306,7 +1316,7 @@ __global__ void __launch_bounds__(kPipeThreads) k_prof_solve_pipe(ProfileSystem 
                                                                   double *xs, double *ds,
                                                                   int backward_only) {
   __shared__ double rv[2][4][kT];
-  volatile int *flags = S.flags;
+  const Waits flags{S.flags, S.wait_ns};
   if (flags[0] != 0) return;                    // the factorisation failed
   const int tid = threadIdx.x;
   const int r = tid >> 3, g = tid & 7;          // tile row, column group (4 columns)

@@ -113,6 +113,7 @@ int ProfileSolver::setup(int n, const int *rowptr, const int *colidx, const int 
   S_.sms = sms;
   S_.counter_bytes = ncount * sizeof(int);
   S_.npairs = npairs_.p; S_.dig = dig_.p;
+  S_.wait_ns = 2000000000ull;
   S_.min_diag_tol = 1.0e-12;   // ProfileSPDLinDirectSolver.h:49 default
   ready_ = true;
   return 0;
