@@ -321,7 +321,8 @@ int xg_profile_get(const xg_model *m, int k, char *name, int cap, double *ms, lo
 
 /* Autotuner (no counterpart in the reference).  what = XG_TUNE_ELEMENT:
    elements per block of the force-based element kernel (1, 2, 4, 8);
-   XG_TUNE_PCG: rows per block of the PCG launch (32..256).  The next
+   XG_TUNE_PCG: rows per block of the PCG launch, node rows where it works on
+   node blocks (32, 64, 128, 256).  The next
    launches of the analysis try the candidates in turn (three timed samples
    each, CUDA events, normalised by fiber state determinations or PCG
    iterations) and keep the cheapest.  Element shapes give bit-identical

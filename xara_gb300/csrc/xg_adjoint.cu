@@ -33,8 +33,10 @@ namespace xg {
 namespace {
 
 // One element (warp) a block, so that a slow element holds up no other's place
-// (1,722 elements in blocks of four and of one: pass A 427 and 389 us, pass B 395
-// and 361, the direct differentiation's 316 and 296, 303 and 282).
+// (in blocks of four and of one: 1,722 elements, pass A 427 and 389 us, pass B 395
+// and 361, the direct differentiation's 316 and 296, 303 and 282; 7,144: 1,484 and
+// 1,462, 1,369 and 1,366, 1,155 and 1,132, 1,099 and 1,096; 29,726: 5,584 and 5,535,
+// 5,160 and 5,136, 4,338 and 4,326, 4,115 and 4,120).
 constexpr int kAdjWarps = 1;
 
 __device__ __forceinline__ double warp_sum_adj(double v) {

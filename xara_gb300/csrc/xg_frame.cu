@@ -1198,15 +1198,14 @@ static void fbc_update_as(const FrameView &v, cudaStream_t s) {
   else k_fbc_update<6, 4, WARPS><<<grid, 32 * WARPS, 0, s>>>(v);
 }
 
-// warps: elements (warps) per block, one of 1, 2, 4, 8 (the autotuner's
-// choice; 4 otherwise), fewer in a model of fewer than 1,024 elements a warp: the
-// elements take unlike numbers of inner iterations, and a block of four keeps its
-// place until its slowest is done, which only many blocks an SM make up for (1,722
-// elements: 97 us in blocks of four, 86 in blocks of one; 88,377: 1,510 and 1,491)
+// warps: elements (warps) per block, 1, 2, 4 or 8 (the autotuner's choice or trial;
+// 1 otherwise).  The elements take unlike numbers of inner iterations, and a larger
+// block keeps its place until its slowest is done.  In blocks of 1, 2, 4, 8: 1,722 2D
+// elements 62, 65, 68, 84 us; 7,144: 181, 189, 189, 204; 88,377: 1,491 in blocks of
+// one, 1,510 of four; 3D, 306: 129, 130, 137, 210; 6,820: 1,044, 1,043, 1,057, 1,112.
 int launch_fbc_update(const FrameView &v, cudaStream_t s, int warps) {
   if (v.ne == 0) return 0;
   if (v.nip > kMaxIp) return XG_EINVAL;
-  while (warps > 1 && v.ne < 1024 * warps) warps >>= 1;
   switch (warps) {
     case 1: fbc_update_as<1>(v, s); break;
     case 2: fbc_update_as<2>(v, s); break;

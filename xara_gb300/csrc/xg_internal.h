@@ -152,10 +152,11 @@ size_t block_ell_bytes(const BlockEll &h, int nblk);
 size_t block_ell_pairs(const BlockEll &h);
 // Solve A x = b (device vectors).  x holds the initial guess (usually 0).
 // Returns 0 when converged, XG_ESOLVE on breakdown, maxit or a barrier timeout.
-// rows_per_block: the grid gets one block per that many rows (capped by
-// co-residency); 0 takes the default of 64
+// rows_per_block: the grid gets one block per that many rows, node rows with the
+// copy (capped by co-residency); 0 takes the default of 64 rows, 32 node rows
 int pcg_solve(const PcgSystem &S, const double *b, double *x, double rtol, int maxit,
               int *iters, double *relres, cudaStream_t s, int rows_per_block = 0);
+int pcg_grid(int n, int nblk, int kb, int rows_per_block, int most);
 int pcg_max_blocks();
 size_t pcg_partial_doubles();
 
@@ -357,7 +358,7 @@ int frame_state_stride(int nip);
 // Concrete02 rows of the device parameter table: the per-material constants
 // into slots 7-11
 int launch_c02_constants(double *uparam, const int *utype, int n, cudaStream_t s);
-int launch_fbc_update(const FrameView &v, cudaStream_t s, int warps = 4);
+int launch_fbc_update(const FrameView &v, cudaStream_t s, int warps = 1);
 int launch_fbc_assemble(const FrameView &v, cudaStream_t s);
 int launch_fbc_commit(const FrameView &v, double *st_c, double *fh_c, long nrec, cudaStream_t s);
 int launch_fbc_revert(const FrameView &v, const double *st_c, long nrec, cudaStream_t s);

@@ -386,7 +386,7 @@ struct xg_model {
   bool step_graph_usable() const;
   int build_step_graph();
   int step_newmark_graph(xg_step_stats *st);
-  int fbc_warps = 4, pcg_rows = 64;
+  int fbc_warps = 1, pcg_rows = 0;        // the autotuner's choices (pcg_rows 0: none)
   cudaEvent_t tune_a = nullptr, tune_b = nullptr;
   // per-kernel CUDA-event timing on the model's stream (xg_profile_*)
   struct ProfSlot {
@@ -2684,7 +2684,8 @@ int xg_autotune_result(const xg_model *m, int *elem_warps, int *pcg_rows_per_blo
                        int *pending) {
   if (!m) return fail(XG_EINVAL, "null model");
   if (elem_warps) *elem_warps = m->fbc_warps;
-  if (pcg_rows_per_block) *pcg_rows_per_block = m->pcg_rows;
+  if (pcg_rows_per_block)
+    *pcg_rows_per_block = m->pcg_rows > 0 ? m->pcg_rows : m->pcg.kb > 0 ? 32 : 64;
   if (pending) *pending = (m->tune_elem.on && !m->tune_elem.done) + (m->tune_pcg.on && !m->tune_pcg.done);
   return 0;
 }

@@ -1307,6 +1307,18 @@ int pcg_factor_blocks(const PcgSystem &S, cudaStream_t s) {
   return 0;
 }
 
+// Blocks of a solve.  Without the copy about four rows per warp: SpMV rows are
+// latency-bound chains (row pointer, column index, vector entry), so mid-size
+// systems want many warps; the grid barrier's cost grows slowly with the block
+// count.  With it a block per SM; small systems fewer, down to a slice of 32 nodes a
+// block (the meetings read every block's slot).
+int pcg_grid(int n, int nblk, int kb, int rows_per_block, int most) {
+  const long rows = kb == 0 ? n : (nblk + 31) / 32;
+  const long per = kb == 0 ? (rows_per_block > 0 ? rows_per_block : 64)
+                           : std::max(rows_per_block / 32, 1);
+  return (int)std::min<long>(std::max<long>((rows + per - 1) / per, 1), most);
+}
+
 // One launch from the x at hand, and with the copy the true residual behind it.
 static int pcg_cycle(const PcgSystem &S, const double *b, double *x, double rtol, int maxit,
                      cudaStream_t s, int rows_per_block, int (&flags)[4], double (&scalars)[8]) {
@@ -1315,21 +1327,14 @@ static int pcg_cycle(const PcgSystem &S, const double *b, double *x, double rtol
   PcgSystem Sv = S;
   void *args[] = {(void *)&Sv, (void *)&b, (void *)&x, (void *)&rtol, (void *)&maxit};
   if (kb == 0) {
-    // about four rows per warp: SpMV rows are latency-bound chains (row
-    // pointer, column index, vector entry), so mid-size systems want many
-    // warps; the grid barrier's cost grows slowly with the block count
-    const long rpb = rows_per_block > 0 ? rows_per_block : 64;
-    const int nb = (int)std::min<long>(std::max<long>(((long)S.n + rpb - 1) / rpb, 1), csr_blocks());
+    const int nb = pcg_grid(S.n, S.nblk, 0, rows_per_block, csr_blocks());
     if (cudaMemsetAsync(S.barrier, 0, 2 * sizeof(unsigned int), s) != cudaSuccess) return XG_ECUDA;
     if (cudaLaunchCooperativeKernel((const void *)k_pcg, dim3(nb), dim3(kPcgThreads), args, 0, s) !=
         cudaSuccess)
       return XG_ECUDA;
   } else {
-    // a block per SM; small systems fewer, down to a slice of 32 nodes a block
-    // (the meetings read every block's slot)
     const long slices = (S.nblk + 31) / 32;
-    const long rpb = rows_per_block > 0 ? std::max<long>(rows_per_block / (32 * kb), 1) : 1;
-    const int nb = (int)std::min<long>(std::max<long>((slices + rpb - 1) / rpb, 1), node_blocks());
+    const int nb = pcg_grid(S.n, S.nblk, kb, rows_per_block, node_blocks());
     const NodeKernel k = kb == 1 ? node_kernel<1>(slices, nb) : kb == 2 ? node_kernel<2>(slices, nb)
                        : kb == 3 ? node_kernel<3>(slices, nb) : node_kernel<6>(slices, nb);
     if (!k.f) return XG_ECUDA;
