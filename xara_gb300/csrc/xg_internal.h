@@ -198,7 +198,7 @@ struct ProfileSystem {
   int nslots;
   int sms;                 // of the device the system lies on
   // right-hand sides whose forward sweep runs inside the factorisation
-  // (fwd_nrhs 0: none)
+  // (1 to 4)
   int fwd_nrhs;
   const double *b[4];      // right-hand sides [n]
   double *x[4];            // solutions [n]

@@ -797,7 +797,6 @@ __device__ bool wait_task(const ProfileSystem &S, int4 t, Waits flags) {
   // row J's forward step: its coupling matrices and the panel tiles of the
   // row further left (the y values of the rows before it are polled inside
   // the step)
-  if (S.fwd_nrhs == 0) return true;
   if (!wait_geq(S.cplq + J, 1, flags)) return false;
   const int ohi = min(S.W, J - S.ftile[J]);
   for (int o = 3; o <= ohi; o++)
@@ -827,7 +826,7 @@ __device__ __forceinline__ double rhs_at(const ProfileSystem &S, int q, int i) {
 }
 
 // Forward substitution of tile row J for the right-hand sides given to the
-// factorisation (S.fwd_nrhs > 0), as a task of the factorisation itself:
+// factorisation (S.fwd_nrhs of them), as a task of the factorisation itself:
 // the right-hand sides are known before the tangent is factored (the
 // unbalance and the reference load of a Newton iteration), so row J's step
 // runs as soon as its coupling matrices are written, a few columns behind
@@ -1270,7 +1269,7 @@ __device__ void worker_block(const ProfileSystem &S, FactorSmem &sm, Waits flags
     else if (t.x == kInverse) inverse_task(S, sm, t.w, tid);
     else if (t.x == kCouple) coupling_task(S, sm, t.w, t.z, tid);
     else if (t.x == kCouple2) second_coupling_task(S, sm, t.w, t.z, tid);
-    else if (S.fwd_nrhs > 0) forward_row(S, t.w, reinterpret_cast<double (*)[kT]>(&sm.A[0][0]), flags);
+    else forward_row(S, t.w, reinterpret_cast<double (*)[kT]>(&sm.A[0][0]), flags);
     csync();
     if (tid == 0) {
       __threadfence();
@@ -1570,7 +1569,7 @@ int profile_device(int *sms) {
 
 int profile_factor(const ProfileSystem &S, cudaStream_t s) {
   if (S.n == 0) return 0;
-  if (S.fwd_nrhs < 0 || S.fwd_nrhs > 4) return XG_EINVAL;
+  if (S.fwd_nrhs < 1 || S.fwd_nrhs > 4) return XG_EINVAL;
   // the sweeps' values: forward ones published inside the factorisation,
   // backward ones by the solve behind it
   const size_t nsweep = 4 * (size_t)S.fwd_nrhs * S.nt * kT;
