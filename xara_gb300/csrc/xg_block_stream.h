@@ -15,8 +15,8 @@ namespace {
 constexpr unsigned long long kCopyTimeoutNs = 2000000000ull;  // 2 s
 
 // By block order: warps a block, blocks a ring stage, stages a warp, stages
-// whose columns' z is gathered ahead.  A stage
-// is one bulk copy of some 2 KB; the rings take most of an SM's shared memory, some 150 KB in flight.
+// whose columns' z is gathered ahead.  A stage is one bulk copy (3,072, 2,304, 2,432
+// and 9,344 bytes), the rings 180 to 192 KiB of an SM's shared memory.
 template <int KB> struct NodeShape;
 template <> struct NodeShape<1> { static constexpr int kWarps = 16, kGroup = 8, kRing = 4, kAhead = 2; };
 template <> struct NodeShape<2> { static constexpr int kWarps = 16, kGroup = 2, kRing = 5, kAhead = 4; };

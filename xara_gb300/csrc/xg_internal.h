@@ -106,13 +106,13 @@ struct PcgSystem {
   // optional node-block sliced ELL copy of the matrix (thread per node row:
   // the equations of one diagonal block against KB x KB blocks of the nodes
   // it couples to, one column index per block) for node rows of at most
-  // nb_cap blocks; the rows of longer node rows in chunks of CSR entries, a
-  // warp each; nb_vals null: every row is read from the CSR arrays warp per
+  // nb_cap blocks; the rows of longer node rows in chunks of CSR entries, four
+  // warps each; nb_vals null: every row is read from the CSR arrays warp per
   // row.  The block SpMV computes in float-float (each value and each entry
   // of z split into two single-precision numbers, xg_ff.h) on the
   // single-precision pipes; node rows with a value outside the split's range
   // stay in FP64.
-  int kb;                 // block order: 2, 3 or 6 (the largest diagonal block), 0: no copy
+  int kb;                 // block order: 1, 2, 3 or 6 (the largest diagonal block), 0: no copy
   const long *nb_off;     // [ceil(nblk/32)+1] slice offsets, in blocks
   const int *nb_cols;     // [nb_off[last]] column node of each block
   const int *nb_len;      // [nblk] blocks of each node row

@@ -567,7 +567,7 @@ __device__ __forceinline__ bool meet(const PcgSystem &S, NodeShared<KB> &E, int 
 // of matrix staying in the L2; from 600,000 on the HBM stream.  Microseconds an
 // iteration, with grid-stride rows, four counting grid barriers and butterflied
 // FP64 sums before: 3,361 equations 47.6, now 13.0; 25,689: 50.5, 19.0; 101,185:
-// 54.3, 26.8; 604,176: 118.7, 103.8 (4.6 TB/s).
+// 54.3, 27.5; 604,176: 118.7, 103.8 (4.6 TB/s).
 template <int KB, int SP, bool kOne>
 __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
     k_pcg_nodes(PcgSystem S, const double *b, double *x, double rtol, int maxit) {

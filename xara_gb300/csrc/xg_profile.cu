@@ -1467,9 +1467,13 @@ int profile_plan(int n, const int *rowptr, const int *colidx, std::vector<int> &
 // column to its last takes a slot of two blocks.  All rows where 28 slots are
 // enough: a row that takes its panels and products from the list needs 14.8 us a
 // column, and the elimination waits for the slowest (one long row behind a
-// constraint held up a 64 x 16 quad block for 150 us).  Beyond that the tile
-// pairs of the list, some 2.7 us each on the blocks that are left, take longer
-// than that a column, and only the two rows next to the diagonal are kept.
+// constraint held up a 64 x 16 quad block for 150 us).  Beyond that only the two rows
+// next to the diagonal are kept: the tile pairs of the list, some 2.7 us each on the
+// blocks that are left, then take longer a column than the rows'.  With all rows
+// kept and with two, us a tile column: 36 below the diagonal tile 14.1 and 15.9, 42
+// 15.2 and 16.4, 49 18.3 and 17.3, 74 148 and 25.2 -- so on 152 SMs the two meet
+// near 45, and the line, which no envelope was measured beyond when it was drawn,
+// lies on the safe side of it.
 // first[I] >= I: no column; rows of a slot in the order of their first columns.
 // A device of fewer SMs than 152 gets its share of the slots, so that blocks for the
 // list are left; two rows next to the diagonal take two slots whatever the system.
