@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <iterator>
@@ -1145,19 +1146,29 @@ __global__ void k_pack_blocks(PcgSystem S) {
 }
 
 // co-resident blocks of the CSR solve; blocks of the node solve (one per SM): of
-// the current device
-int sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
+// the current device (its occupancy, a slow query, asked once)
+int sm_count(int dev) {
+  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms;
 }
 int csr_blocks() {
-  int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg, kPcgThreads, 0);
-  return sm_count() * std::max(per, 1);
+  static std::atomic<int> known[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int per = dev < 64 ? known[dev].load() : 0;
+  if (per == 0) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg, kPcgThreads, 0);
+    per = std::max(per, 1);
+    if (dev < 64) known[dev].store(per);
+  }
+  return sm_count(dev) * per;
 }
-int node_blocks() { return std::min(sm_count(), kPcgMaxBlocks); }
+int node_blocks() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return std::min(sm_count(dev), kPcgMaxBlocks);
+}
 
 struct NodeKernel {
   const void *f;
@@ -1343,7 +1354,7 @@ static int pcg_cycle(const PcgSystem &S, const double *b, double *x, double rtol
     if (cudaLaunchCooperativeKernel(k.f, dim3(nb), dim3(k.threads), args, k.smem, s) != cudaSuccess)
       return XG_ECUDA;
     const int rows = kResidualThreads / 32;
-    const int rb = (int)std::min<long>(((long)S.n + rows - 1) / rows, pcg_partial_doubles());
+    const int rb = (int)std::min<long>(((long)S.n + rows - 1) / rows, 12 * node_blocks());
     k_pcg_residual<<<rb, kResidualThreads, 0, s>>>(S, b, x);
     if (cudaGetLastError() != cudaSuccess) return XG_ECUDA;
   }
