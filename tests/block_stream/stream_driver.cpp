@@ -84,26 +84,29 @@ static int run(int ns, int stride, int passes, int lose, unsigned seed) {
     Stream B{S, reinterpret_cast<Record(*)[kGroup]>(ring.data()), full, 0, part, 0, kOne ? ns : stride,
              last};
     B.start();
+    bool ok = true;
     for (int it = 0; it < passes; it++)
       for (int s = 0; s < last; s += kOne ? ns : stride) {
         const int width = B.width(s), groups = kOne ? B.total : B.groups(width);
         auto gather = [&](int g) {
           if (g >= groups) return;
-          const Record *r = B.get();
-          g_failed = B.lost();
+          const Record *r = B.get(ok);
+          g_failed = !ok;
           for (int u = 0; u < kGroup; u++) {
             const int k = kGroup * (part + SP * g) + u;
-            if (k < width && r[u].col[0] != (B.lost() ? 0 : (int)(off[s] / 32) + k)) errors++;
+            if (k >= width) continue;
+            const int col = r[u].col[0];               // a record's or, of a lost one, node 0
+            errors += ok ? col != (int)(off[s] / 32) + k : col < 0 || col > nrec;
           }
         };
         for (int u = 0; u < kAhead; u++) gather(u);
         for (int g = 0; g < groups; g += kAhead)
           for (int u = 0; u < kAhead && g + u < groups; u++) {
-            B.release();
+            B.release(ok);
             gather(g + u + kAhead);
           }
       }
-    if (lose < 0 && B.lost()) errors++;
+    if (lose < 0 && !ok) errors++;
     B.drain();
     for (auto &b : g_bar)
       if (b.second.armed != b.second.done && !b.second.lost) errors++;   // still on its way

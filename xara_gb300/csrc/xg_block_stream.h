@@ -73,51 +73,18 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *b, unsigned parity)
 // iteration's blocks is there when its z is.  A share no longer than the ring
 // is loaded once.  Lane 0 issues.
 //
-// A copy that has not come within the limit ends the stream: what lies in its
-// stage is no record (its columns would send the gathers anywhere), so the ring's
-// columns become node 0 and no wait follows; no stage is filled again, and the
-// other copies in flight are waited for, all within one limit more.
-__device__ inline bool wait_until(unsigned long long *b, unsigned parity, unsigned long long end) {
-  for (int k = 0;; k++) {
-    if (mbar_try(b, parity)) return true;
-    if ((k & 63) == 63 && global_ns() > end) return false;
-  }
-}
-// from stage next on (a ring's groups taken and not yet released have come)
-__device__ __noinline__ void ring_drain(unsigned long long *full, int next, int oldest, int len,
-                                        unsigned phase, bool ring) {
-  const unsigned long long end = global_ns() + kCopyTimeoutNs;
-  for (int k = ring ? (next - oldest + len) % len : 0; k < len; k++) {
-    wait_until(full + next, phase, end);
-    if (++next == len) {
-      next = 0;
-      phase ^= (unsigned)ring;
-    }
-  }
-}
-// false when the ring is over: stage next has not come
-template <int KB>
-__device__ __noinline__ bool ring_wait(unsigned long long *full,
-                                       BlockRecord<KB> (*rec)[NodeShape<KB>::kGroup], int lane,
-                                       int next, int oldest, int len, unsigned phase, bool ring) {
-  constexpr int kRing = NodeShape<KB>::kRing;
-  volatile unsigned long long *lost = full + kRing;
-  if (*lost) return false;
-  if (wait_until(full + next, phase, global_ns() + kCopyTimeoutNs)) return ring;
-  if (lane == 0) ring_drain(full, next, oldest, len, phase, ring);
-  for (int s = 0; s < kRing; s++)
-    for (int u = 0; u < NodeShape<KB>::kGroup; u++) rec[s][u].col[lane] = 0;
-  *lost = 1;
-  return false;
-}
-
+// A copy that has not come within the limit ends the stream (ok, the warp's own):
+// what lies in its stage is no record (its columns would send the gathers
+// anywhere), so the stage's columns become node 0, and no wait follows; no stage is
+// filled again, and drain() waits for the copies still in flight, all within one
+// limit more.
 template <int KB, int SP, bool kOne>
 struct BlockStream {
   static constexpr int kGroup = NodeShape<KB>::kGroup, kRing = NodeShape<KB>::kRing;
   using Record = BlockRecord<KB>;
   const PcgSystem &S;
   Record (*rec)[kGroup];        // the warp's ring
-  unsigned long long *full;     // a barrier a stage, then whether a copy was lost
+  unsigned long long *full;     // a barrier a stage, then where lane 0 lost a copy
   int lane, part, first, stride, ns;
   int total, len;               // groups of the share, stages in use
   bool ring;                    // more groups than stages
@@ -154,11 +121,11 @@ struct BlockStream {
     phase = 0u;
     if (total > 0) {
       next_slice(first);
-      for (int k = 0; k < len; k++) issue(k);
+      for (int k = 0; k < len; k++) issue(k, true);
     }
   }
-  __device__ __forceinline__ void issue(int k) {
-    if (lane == 0) {
+  __device__ __forceinline__ void issue(int k, bool ok) {
+    if (lane == 0 && ok) {
       const unsigned bytes =
           (unsigned)sizeof(Record) * (kGroup == 1 ? 1u : (unsigned)min(kGroup, wide));
       mbar_expect(full + k, bytes);
@@ -177,14 +144,11 @@ struct BlockStream {
     }
   }
   // the next group, once it has come
-  __device__ __forceinline__ const Record *get() {
-    if (!mbar_try(full + next, phase)) wait();
+  __device__ __forceinline__ const Record *get(bool &ok) {
+    ok &= wait(ok);
     const Record *r = rec[next];
     advance();
     return r;
-  }
-  __device__ __forceinline__ bool lost() const {
-    return *(const volatile unsigned long long *)(full + kRing) != 0;
   }
   __device__ __forceinline__ void advance() {
     if (++next == len) {
@@ -193,18 +157,43 @@ struct BlockStream {
     }
   }
   // the warp is done with the oldest group
-  __device__ __forceinline__ void release() {
+  __device__ __forceinline__ void release(bool ok) {
     __syncwarp();
-    if (ring) issue(oldest);
+    if (ring) issue(oldest, ok);
     if (++oldest == len) oldest = 0;
   }
-  __device__ __forceinline__ void wait() {
-    if (!ring_wait<KB>(full, rec, lane, next, oldest, len, phase, ring)) ring = false;
+  __device__ __forceinline__ bool wait(bool ok) {
+    unsigned long long t0 = 0;
+    for (int tries = 0;; tries++) {
+      if (mbar_try(full + next, phase)) return true;
+      if (ok) {
+        if ((tries & 63) != 63) continue;
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 <= kCopyTimeoutNs) continue;
+        if (lane == 0)
+          full[kRing] = 1u | (unsigned)next << 8 | (unsigned)oldest << 16 | phase << 24;
+      }
+      for (int u = 0; u < kGroup; u++) rec[next][u].col[lane] = 0;
+      return false;
+    }
   }
   // the copies in flight have come: nothing may land after the block is gone
-  __device__ __forceinline__ void drain() {
-    if (lane == 0 && len > 0 && full[kRing] == 0)
-      ring_drain(full, next, oldest, len, phase, ring);
+  __device__ void drain() {
+    if (lane != 0 || len == 0) return;
+    if (full[kRing] != 0) {          // as lane 0 stood when it lost one
+      const unsigned at = (unsigned)full[kRing];
+      next = at >> 8 & 255u;
+      oldest = at >> 16 & 255u;
+      phase = at >> 24 & 1u;
+    }
+    // (a ring's groups taken and not yet released have come)
+    const unsigned long long end = global_ns() + kCopyTimeoutNs;
+    for (int k = ring ? (next - oldest + len) % len : 0; k < len; k++) {
+      for (int t = 0; !mbar_try(full + next, phase); t++)
+        if ((t & 63) == 63 && global_ns() > end) break;
+      advance();
+    }
   }
 };
 

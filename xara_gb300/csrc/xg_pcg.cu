@@ -815,7 +815,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
         // z of the columns of group g
         auto gather = [&](int g, float2 (&o)[kGroup][KS]) {
           if (g >= groups) return;
-          const BlockRecord<KB> *r = blocks.get();
+          const BlockRecord<KB> *r = blocks.get(ok);
 #pragma unroll
           for (int u = 0; u < kGroup; u++)
             if (kGroup == 1 || kGroup * (part + SP * g) + u < width)
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
 #pragma unroll
               for (int c = 0; c < KB; c++) ff_madd(r[u].v[a * KB + c][lane], zz[u][c], h[a], l[a]);
           }
-          blocks.release();
+          blocks.release(ok);
         };
         float2 zg[kAhead][kGroup][KS];
 #pragma unroll
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(32 * NodeShape<KB>::kWarps, 1)
           if (L.in) lpq += beta * S.q[L.row] * (S.z[L.row] + beta * S.p[L.row]);
         });
       }
-      if (blocks.lost()) {         // a copy that did not come
+      if (!ok) {         // a copy that did not come
         flags[0] = 2;
         E.ok[epoch & 1] = 0;
       }
