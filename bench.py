@@ -797,9 +797,8 @@ def run_batch(args):
                      "frac": achieved / peak if achieved and peak else None,
                      "peak_source": peak_kind, "traffic": ncu_traffic("batch", dominant),
                      "algorithmic_bytes_per_launch": alg,
-                     "limit": "the FP64 pipe, not HBM: 78.6 % active under ncu "
-                              "(profiles/k_fbc_update_batch_c3.md); the fraction above is the "
-                              "kernel's HBM view"},
+                     "limit": "the FP64 pipe, not HBM: 78.6 % active under ncu; "
+                              "the fraction above is the kernel's HBM view"},
         "kernels_ms_per_step": {k: v[0] / args.steps for k, v in kernels.items()},
         "clocks": clocks,
         "setup_s": t_setup,
@@ -1415,7 +1414,7 @@ def run_brick(args):
                      "algorithmic_bytes_per_launch": alg.get(dominant, alg["phase"]),
                      "limit": "instruction issue on the single-precision pipes, not HBM: the "
                               "tangent's float-float sums (IPC 2.9 of 4, FMA pipe 53 % under "
-                              "ncu: profiles/k_brick_assemble_brick_c2_small.md)"},
+                              "ncu)"},
         "fp64": {"est_flops_per_step": flops, "achieved_tflops": flops / phase_s / 1e12,
                  "peak_tflops_probe": fp64_peak,
                  "frac": (flops / phase_s / 1e12) / fp64_peak if fp64_peak else None},
